@@ -10,303 +10,333 @@
 //   non-KB step i : acc += round(IFFNT(sum_r FFNT(dec_r(X^abar acc - acc)) BK_i[r]))
 //   KB pair p     : acc  = round(IFFNT(sum_r FFNT(dec_r(acc)) KB_p[r])),
 //                   KB = H + bk0 (X^{a0+a1}-1) + bk1 (X^{a0}-1) + bk2 (X^{a1}-1).
+// The H term of a KeyBundle step adds the value of the digits; it is added as
+// an integer after the rounding, (acc + 2^15) & 0xffff0000, instead of through
+// the transforms.
 //
-// B200 layout.  One CTA carries G lanes (gates) through every step in
-// lockstep, so each Fourier-domain key row read from L2 serves G gates
-// (the reference reads the whole key per gate).  4 warps per lane:
-//   phase 1  warp (g, r): digits of row r of lane g, fold + twist, forward
-//            512-point FFT (one warp per transform, fft64.cuh) -> spec[g][r]
-//   phase 2  thread f (frequency bin): key multiply-accumulate for all G lanes;
-//            key words are read once per CTA with 128-bit loads; the KeyBundle
-//            factors X^a - 1 are evaluated from a 2N-entry root table
-//            (psi^{(1+4f) a} - 1) instead of the reference's 16 MB xai table
-//   phase 3  warp (g, j): inverse FFT, untwist, round, write acc[g][j]
-// Epilogue: SampleExtract straight from shared memory to the lane output.
-// Batches of up to 16 lanes run the latency form k_br_fp64_clu instead: one
-// lane per cluster of four CTAs on four SMs, each multiplying a quarter of the
-// bins with the key (a lone lane is bound by one SM's L2 bandwidth for the
-// 196 KB of key rows per step) and gathering the other quarters through
-// distributed shared memory for the inverse transforms.
+// Two forms, by the number of lanes (gates) per SM:
+//   k_br_fp64      two lanes per CTA, one warp per polynomial: batches that
+//                  fill the GPU
+//   k_br_fp64_one  one lane per CTA or per cluster of four CTAs, two warps per
+//                  digit row: up to three lanes per SM
+// A step is, in both: forward transforms of the digits -> spectra in shared
+// memory | multiply-accumulate with the key, bin by bin | inverse transforms,
+// rounding.  At lvl1 the rounded values are the exact integers (products below
+// 2^44 against 53 bits), so every form gives the same words.
+//
+// What bounds it: the FP64 pipe takes a warp's fused multiply-add in two
+// cycles, but an instruction with three register operands needs three (43
+// against 63 per clock and SM measured; two register operands and a constant
+// run at full rate).  A KeyBundle step is 154 K FP64 operations per lane, 62 K
+// of them the products with three register operands; counted with their
+// operands a lane step cannot take less than 3.4 K cycles of an SM.  4789
+// lanes: 26.9 -> 23.3 ms (4.5 K cycles); plain key 42.0 -> 38.4 ms.
 #include <stdlib.h>
 
 #include <cooperative_groups.h>
 
 #include "engine.h"
-#include "fft64.cuh"
+#include "ffnt_tree16.cuh"
 
 namespace cufhe {
 
 namespace {
 
-constexpr int kDefaultBrGates = 2;
-constexpr int kAbarStride = 640;
 constexpr uint32_t kDecOffset = (128u << 24) + (128u << 16) + (1u << 15);  // offsetgen + round
+constexpr int kRootEntries = 514;  // psi^t, t <= 512, padded to an even count
 
-template <int G>
-constexpr size_t br_smem_bytes()
+// Shared-memory position of psi^t (t in [0, 512]): the low 3 bits XORed with
+// the next 3, so that the strided gathers psi^{(1 + 4 f) a} spread over the
+// banks.
+__device__ __forceinline__ int root_pos(uint32_t t) { return (int)(t ^ ((t >> 3) & 7u)); }
+
+// psi^t for any t (mod 2N): psi^512 = i
+__device__ __forceinline__ double2 root_at(const double2* tab, uint32_t t)
 {
-    return sizeof(double2) * G * 4 * kSlotStride + sizeof(double2) * kN +
-           sizeof(uint32_t) * G * kTrlwe + sizeof(uint16_t) * G * kAbarStride;
+    double2 v = tab[root_pos(t & 511u)];
+    if (t & 512u) v = make_double2(-v.y, v.x);
+    if (t & 1024u) v = make_double2(-v.x, -v.y);
+    return v;
 }
 
-// Word of coefficient n (0 <= n < 2N) of a lane's accumulator in shared
-// memory.  The KeyBundle form flips bit 4 when bit 7 is set: the inverse
-// transforms store coefficients n and n + 128 from lanes l and l + 16 in one
-// instruction, which would otherwise fall in the same bank; the forward
-// transforms' reads of 32 consecutive coefficients stay conflict-free.  (The
-// plain form keeps the natural order: its rotated reads X^a acc start
-// anywhere.)
+// i^m v (exact)
+__device__ __forceinline__ double2 mul_ipow(double2 v, uint32_t m)
+{
+    if (m & 1u) v = make_double2(-v.y, v.x);
+    if (m & 2u) v = make_double2(-v.x, -v.y);
+    return v;
+}
+
+// The gadget needs only the upper halves of acc + kDecOffset: digit 0 (most
+// significant) is byte 1 of a half minus 128, digit 1 byte 0 minus 128, and
+// the value the digits stand for is (half - 0x8080) << 16.  A thread keeps
+// coefficient n's half in the lower and n + 512's in the upper 16 bits.
+__device__ __forceinline__ uint32_t pack_halves(uint32_t lo, uint32_t hi)
+{
+    return ((lo + kDecOffset) >> 16) | ((hi + kDecOffset) & 0xffff0000u);
+}
+__device__ __forceinline__ double2 digits_of(uint32_t h, int d)
+{
+    const int sh = 8 - 8 * d;
+    return make_double2(small_to_double((h >> sh) & 255u, 128),
+                        small_to_double((h >> (16 + sh)) & 255u, 128));
+}
+__device__ __forceinline__ uint32_t recompose_lo(uint32_t h) { return (h << 16) - 0x80800000u; }
+__device__ __forceinline__ uint32_t recompose_hi(uint32_t h) { return (h & 0xffff0000u) - 0x80800000u; }
+
+// coefficient i of the test vector X^bar (mu + mu X + ..)
+__device__ __forceinline__ uint32_t test_coef(uint32_t bar, uint32_t i, uint32_t mu)
+{
+    if (bar == 2u * kN) return mu;
+    return ((i < (bar & (kN - 1))) ^ (bar >> 10)) ? 0u - mu : mu;
+}
+
+// CTAs of a grid that all run at once and share the work of prefetching
+constexpr unsigned kPrefetchCtas = 444;
+
+
+// ---- two lanes per CTA, one warp per polynomial.
+// The warp keeps its polynomial's digits in registers from the rounding of a
+// step to the transforms of the next (KeyBundle; the plain form rotates the
+// accumulator and keeps it in shared memory), so a step has two barriers and
+// no warp idles in the inverse transforms.  Three CTAs per SM (168 registers,
+// 76 KB): six lanes whose phases drift apart, so that one CTA's key loads run
+// under the others' transforms.  4789 lanes KeyBundle: 23.3 ms; two CTAs per
+// SM with the registers that leaves 25.2 ms, but 3.18 against 3.24 ms for 592
+// lanes, which is one round of them.  Measured and not kept: neighbouring
+// threads sharing a bin, one output polynomial each, with the key words of the
+// next bin loaded ahead (25.5 ms); eight lanes per SM whose spectra stay in
+// tensor memory (24.9 ms for 4736); six lanes in one CTA (31.5 ms); 8 points
+// per thread and twice the warps (28.4 ms); the transforms' twiddles in shared
+// memory instead of the L1 (25.5 against 24.6 ms).
 template <bool KB>
-__device__ __forceinline__ int acc_ix(int n)
+constexpr size_t two_smem_bytes()
 {
-    return KB ? n ^ (((n >> 7) & 1) << 4) : n;
+    return sizeof(double2) * (2 * 4 * kHalfN + (KB ? kRootEntries : 0)) +
+           (KB ? 0 : sizeof(uint32_t) * 2 * kTrlwe) + sizeof(uint16_t) * 2 * kN0;
 }
+static_assert(two_smem_bytes<true>() <= 76800, "three KeyBundle CTAs per SM");
+static_assert(two_smem_bytes<false>() <= 113 * 1024, "two plain CTAs per SM");
 
-// signed digit d (0 = most significant) of an offset Torus32 value
-__device__ __forceinline__ double digit_of(uint32_t t, int d)
+template <bool KB, int MINB>
+__global__ void __launch_bounds__(128, MINB)
+    k_br_fp64(const uint32_t* __restrict__ lane_in, int lanes, uint32_t mu,
+              const double2* __restrict__ bkf, const double2* __restrict__ psi, int steps,
+              uint32_t* __restrict__ acc_out, uint32_t* __restrict__ lane_out)
 {
-    return (double)((int32_t)((t >> (24 - 8 * d)) & 255u) - 128);
-}
-
-template <bool KB, int G>
-__global__ void __launch_bounds__(G * 128, G == 1 ? 3 : (G == 2 ? 2 : 1)) k_br_fp64(const uint32_t* __restrict__ lane_in, int lanes,
-                                                     uint32_t mu, const double2* __restrict__ bkf,
-                                                     const double2* __restrict__ psi,
-                                                     const double2* __restrict__ tw512, int steps,
-                                                     uint32_t* __restrict__ acc_out,
-                                                     uint32_t* __restrict__ lane_out)
-{
+    constexpr int G = 2, NT = 128;
+    constexpr int E = KB ? 3 : 1;               // keys per step
+    constexpr size_t kTrgswF = 4 * 2 * kHalfN;  // double2 per Fourier TRGSW
     extern __shared__ __align__(16) unsigned char smem[];
-    double2* spec = reinterpret_cast<double2*>(smem);
-    double2* psi_s = spec + G * 4 * kSlotStride;  // root table, interleaved (psi_pos)
-    uint32_t* acc = reinterpret_cast<uint32_t*>(psi_s + kN);
-    uint16_t* abar = reinterpret_cast<uint16_t*>(acc + G * kTrlwe);
+    double2* spec = reinterpret_cast<double2*>(smem);  // [G][4][512]
+    double2* roots = spec + G * 4 * kHalfN;            // KeyBundle only
+    uint32_t* acc = reinterpret_cast<uint32_t*>(roots + (KB ? kRootEntries : 0));  // plain only
+    uint16_t* abar = reinterpret_cast<uint16_t*>(acc + (KB ? 0 : G * kTrlwe));
+    const double2* const ltw = psi + kTw16At;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int lane_base = blockIdx.x * G;
+    const int wg = warp >> 1, wj = warp & 1;
+    const int low = tree_low(lane);
 
-    for (int t = tid; t < kN; t += blockDim.x) psi_s[psi_pos((uint32_t)t)] = psi[t];
-    // ---- prologue: modulus switch and test vector (RotatedTestVector)
-#pragma unroll 1
+    if (KB)
+        for (int t = tid; t <= 512; t += NT) roots[root_pos((uint32_t)t)] = psi[t];
     for (int g = 0; g < G; g++) {
         const int l = lane_base + g;
         const bool ok = l < lanes;
         const uint32_t* x = lane_in + (size_t)(ok ? l : 0) * kTlwe0;
-        for (int i = tid; i < kN0; i += blockDim.x)
-            abar[g * kAbarStride + i] = ok ? (uint16_t)((x[i] + (1u << 20)) >> 21) : 0;
-        const uint32_t bar = ok ? 2u * kN - (x[kN0] >> 21) : 2u * kN;
-        for (int i = tid; i < kN; i += blockDim.x) {
-            acc[g * kTrlwe + acc_ix<KB>(i)] = 0;
-            uint32_t v;
-            if (bar == 2u * kN)
-                v = mu;
-            else
-                v = (((uint32_t)i < (bar & (kN - 1))) ^ (bar >> 10)) ? 0u - mu : mu;
-            acc[g * kTrlwe + acc_ix<KB>(kN + i)] = v;
+        for (int i = tid; i < kN0; i += NT)
+            abar[g * kN0 + i] = ok ? (uint16_t)((x[i] + (1u << 20)) >> 21) : 0;
+    }
+    const int total = KB ? kN0 / 2 : kN0;
+    const int nsteps = (steps < 0 || steps > total) ? total : steps;
+    // this warp's polynomial; KeyBundle: the accumulators land in the spectra's
+    // place after the last step
+    uint32_t* const own = (KB ? reinterpret_cast<uint32_t*>(spec) : acc) + (wg * 2 + wj) * kN;
+    uint32_t P[16];
+    {
+        const int l = lane_base + wg;
+        const uint32_t bar = l < lanes ? 2u * kN - (lane_in[(size_t)l * kTlwe0 + kN0] >> 21) : 2u * kN;
+#pragma unroll
+        for (int m = 0; m < 16; m++) {
+            const uint32_t n = (uint32_t)(low + 32 * m);
+            const uint32_t lo = wj ? test_coef(bar, n, mu) : 0u, hi = wj ? test_coef(bar, n + 512, mu) : 0u;
+            if (!KB || nsteps == 0) {
+                own[n] = lo;
+                own[n + 512] = hi;
+            }
+            P[m] = pack_halves(lo, hi);
         }
     }
     __syncthreads();
 
-    const int total = KB ? kN0 / 2 : kN0;
-    const int nsteps = (steps < 0 || steps > total) ? total : steps;
-    constexpr size_t kTrgswF = 4 * 2 * kHalfN;  // double2 per Fourier TRGSW
+    double2* const slot = spec + (wg * 4 + 2 * wj) * kHalfN;
+    const int sl = spec16_lane(lane);
 
 #pragma unroll 1
     for (int p = 0; p < nsteps; p++) {
-        // ---- phase 1: decompose + fold + twist + forward FFT, warp (g, r)
-        {
-            const int g = warp >> 2, r = warp & 3, j = r >> 1, d = r & 1;
-            const uint32_t* a = acc + g * kTrlwe + j * kN;
-            double2 v[16];
-            const uint32_t ab = KB ? 0u : abar[g * kAbarStride + p];
-            const uint32_t abm = ab & (kN - 1), abn = ab >> 10;
+        if (tid == 0 && p + 2 < nsteps && gridDim.x <= kPrefetchCtas)
+            prefetch_part(bkf + (size_t)(p + 2) * E * kTrgswF, E * kTrgswF * sizeof(double2),
+                          blockIdx.x, gridDim.x);
+        if (!KB) {
+            // X^abar acc - acc (include/gatebootstrapping_gpu.cuh:114-138)
+            const uint32_t ab = abar[wg * kN0 + p], abm = ab & (kN - 1), abn = ab >> 10;
 #pragma unroll
-            for (int n2 = 0; n2 < 16; n2++) {
-                const int n = lane + 32 * n2;
-                uint32_t lo = a[acc_ix<KB>(n)], hi = a[acc_ix<KB>(n + kHalfN)];
-                if (!KB) {
-                    // X^abar acc - acc (include/gatebootstrapping_gpu.cuh:114-138)
-                    uint32_t rl = a[(n - ab) & (kN - 1)];
-                    uint32_t rh = a[(n + kHalfN - ab) & (kN - 1)];
-                    rl = (((uint32_t)n < abm) ^ abn) ? 0u - rl : rl;
-                    rh = (((uint32_t)(n + kHalfN) < abm) ^ abn) ? 0u - rh : rh;
-                    lo = rl - lo;
-                    hi = rh - hi;
-                }
-                v[n2] = make_double2(digit_of(lo + kDecOffset, d), digit_of(hi + kDecOffset, d));
+            for (int m = 0; m < 16; m++) {
+                const uint32_t n = (uint32_t)(low + 32 * m);
+                uint32_t rl = own[(n - ab) & (kN - 1)], rh = own[(n + 512 - ab) & (kN - 1)];
+                rl = ((n < abm) ^ abn) ? 0u - rl : rl;
+                rh = ((n + 512 < abm) ^ abn) ? 0u - rh : rh;
+                P[m] = pack_halves(rl - own[n], rh - own[n + 512]);
             }
-            double2* slot = spec + (g * 4 + r) * kSlotStride;
-            ffnt_forward_warp(v, slot, psi_s, lane);
-#pragma unroll
-            for (int q = 0; q < 16; q++) slot[ffnt_pos(lane, q)] = v[q];
         }
-        __syncthreads();
-
-        // ---- phase 2: key multiply-accumulate, thread f = frequency bin.
-        // One (bin, output polynomial) item at a time with all twelve key
-        // words of the item (rows x keys) loaded before any is used: the
-        // phase is bound by the latency of the key rows from L2, and this
-        // keeps 12 loads per thread in flight (a rows-outermost loop with both
-        // outputs' accumulators live leaves room for only one row's 6).  The
-        // output of polynomial 0 overwrites row 0's spectrum, which polynomial
-        // 1 still reads, so it is held in registers until both are done.  Per
-        // bin and output the additions run in the same order as in
-        // k_br_fp64_clu (rows 0..3, then H, x01, x0, x1): bit-identical.
-        if (KB) {
-            const double2* bk = bkf + (size_t)p * 3 * kTrgswF;
-            // KeyBundle roots psi^{(1 + 4 f) a} (a = a0 + a1, a0, a1) of the
-            // thread's first bin.  With two lanes per CTA the thread's bins
-            // are f and f + 256, and psi^{(1 + 4 (f + 256)) a} = (-1)^a
-            // psi^{(1 + 4 f) a} exactly (a sign flip), so the roots are
-            // gathered once per step; the table gathers are bank-conflicted
-            // for even a.  Other lane counts gather per bin.
-            double2 root[G][3];
-            uint32_t odd[G];
-            if (G == 2) {
-                const uint32_t ef = 1u + 4u * (uint32_t)tid;
-#pragma unroll
-                for (int g = 0; g < G; g++) {
-                    const uint32_t a0 = abar[g * kAbarStride + 2 * p];
-                    const uint32_t a1 = abar[g * kAbarStride + 2 * p + 1];
-                    root[g][0] = psi_at(psi_s, ef * (a0 + a1));
-                    root[g][1] = psi_at(psi_s, ef * a0);
-                    root[g][2] = psi_at(psi_s, ef * a1);
-                    odd[g] = (((a0 + a1) & 1u) << 0) | ((a0 & 1u) << 1) | ((a1 & 1u) << 2);
-                }
-            }
+        // ---- forward transforms of both digits of this warp's polynomial
 #pragma unroll 1
-            for (int f = tid; f < kHalfN; f += blockDim.x) {
-                const uint32_t ef = 1u + 4u * (uint32_t)f;
-                double2 o0[G];
+        for (int d = 0; d < 2; d++) {
+            double2 v[16];
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    double2 b[4][3];
+            for (int n = 0; n < 16; n++) v[n] = digits_of(P[n], d);
+            tree16_forward(v, slot + d * kHalfN, ltw, lane);
 #pragma unroll
-                    for (int r = 0; r < 4; r++)
+            for (int q = 0; q < 16; q++) slot[d * kHalfN + sl + 32 * tree_pos(q)] = v[q];
+        }
+
+        // ---- key multiply-accumulate, thread = bins tid + 128 i.  The key
+        // words of the two output polynomials lie side by side (one 256-bit
+        // load); one key at a time keeps four of them in flight per thread
+        // beside both lanes' spectra and sums.  The KeyBundle roots of the
+        // bins 128 apart follow from the first's: psi^{512 a} = i^a (exact).
+        {
+            const double2* bk = bkf + (size_t)p * E * kTrgswF + 2 * tid;
+            double2 root[G][3];
+            uint32_t rot[G];
+            if constexpr (KB) {
+                const uint32_t ex = 1u + 4u * (uint32_t)tid;
 #pragma unroll
-                        for (int e = 0; e < 3; e++)
-                            b[r][e] = __ldg(&bk[((e * 4 + r) * 2 + j) * kHalfN + f]);
-#pragma unroll
-                    for (int g = 0; g < G; g++) {
-                        double2 D[4], sum[3];
-#pragma unroll
-                        for (int r = 0; r < 4; r++) D[r] = spec[(g * 4 + r) * kSlotStride + f];
-#pragma unroll
-                        for (int r = 0; r < 4; r++)
-#pragma unroll
-                            for (int e = 0; e < 3; e++)
-                                sum[e] = r == 0 ? cfma(make_double2(0.0, 0.0), D[r], b[r][e])
-                                                : cfma(sum[e], D[r], b[r][e]);
-                        // FFNT(H 2^-32) = 2^-8 (d = 0), 2^-16 (d = 1) on poly j
-                        double2 o = make_double2(fma(D[2 * j].x, 0x1p-8, D[2 * j + 1].x * 0x1p-16),
-                                                 fma(D[2 * j].y, 0x1p-8, D[2 * j + 1].y * 0x1p-16));
-                        double2 x01, x0, x1;
-                        if (G == 2) {
-                            x01 = root[g][0];
-                            x0 = root[g][1];
-                            x1 = root[g][2];
-                        } else {
-                            const uint32_t a0 = abar[g * kAbarStride + 2 * p];
-                            const uint32_t a1 = abar[g * kAbarStride + 2 * p + 1];
-                            x01 = psi_at(psi_s, ef * (a0 + a1));
-                            x0 = psi_at(psi_s, ef * a0);
-                            x1 = psi_at(psi_s, ef * a1);
-                        }
-                        x0.x -= 1.0;
-                        x1.x -= 1.0;
-                        x01.x -= 1.0;
-                        o = cfma(o, x01, sum[0]);
-                        o = cfma(o, x0, sum[1]);
-                        o = cfma(o, x1, sum[2]);
-                        if (j == 0) {
-                            o0[g] = o;
-                        } else {
-                            spec[(g * 4 + 0) * kSlotStride + f] = o0[g];
-                            spec[(g * 4 + 1) * kSlotStride + f] = o;
-                        }
-                    }
-                }
-                if (G == 2) {
-#pragma unroll
-                    for (int g = 0; g < G; g++)
-#pragma unroll
-                        for (int e = 0; e < 3; e++)
-                            if ((odd[g] >> e) & 1u) {
-                                root[g][e].x = -root[g][e].x;
-                                root[g][e].y = -root[g][e].y;
-                            }
+                for (int g = 0; g < G; g++) {
+                    const uint32_t a0 = abar[g * kN0 + 2 * p], a1 = abar[g * kN0 + 2 * p + 1];
+                    root[g][0] = root_at(roots, ex * (a0 + a1));
+                    root[g][1] = root_at(roots, ex * a0);
+                    root[g][2] = root_at(roots, ex * a1);
+                    rot[g] = (a0 & 3u) | ((a1 & 3u) << 2);
                 }
             }
-        } else {
-            const double2* bk = bkf + (size_t)p * kTrgswF;
-            for (int f = tid; f < kHalfN; f += blockDim.x) {
-                double2 o[G][2];
+            __syncthreads();
+            const int ix0 = spec16_ix(tid);
+#pragma unroll 1
+            for (int i = 0; i < 4; i++) {
+                const int ix = ix0 + 128 * i;
+                double2 D[G][4], o[G][2];
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    double2 b[2];
+                for (int g = 0; g < G; g++) {
+                    o[g][0] = o[g][1] = make_double2(0.0, 0.0);
 #pragma unroll
-                    for (int j = 0; j < 2; j++) b[j] = __ldg(&bk[(r * 2 + j) * kHalfN + f]);
+                    for (int r = 0; r < 4; r++) D[g][r] = spec[(g * 4 + r) * kHalfN + ix];
+                }
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    double2 k[4][2];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) key_pair(k[r][0], k[r][1], &bk[(e * 4 + r) * 1024 + i * 256]);
 #pragma unroll
                     for (int g = 0; g < G; g++) {
-                        const double2 D = spec[(g * 4 + r) * kSlotStride + f];
+                        double2 s0 = cfma(make_double2(0.0, 0.0), D[g][0], k[0][0]);
+                        double2 s1 = cfma(make_double2(0.0, 0.0), D[g][0], k[0][1]);
 #pragma unroll
-                        for (int j = 0; j < 2; j++)
-                            o[g][j] = r == 0 ? cfma(make_double2(0.0, 0.0), D, b[j])
-                                             : cfma(o[g][j], D, b[j]);
+                        for (int r = 1; r < 4; r++) {
+                            s0 = cfma(s0, D[g][r], k[r][0]);
+                            s1 = cfma(s1, D[g][r], k[r][1]);
+                        }
+                        if constexpr (KB) {
+                            double2 x = root[g][e];
+                            x.x -= 1.0;
+                            o[g][0] = cfma(o[g][0], x, s0);
+                            o[g][1] = cfma(o[g][1], x, s1);
+                        } else {
+                            o[g][0] = s0;
+                            o[g][1] = s1;
+                        }
                     }
                 }
 #pragma unroll
                 for (int g = 0; g < G; g++) {
-                    spec[(g * 4 + 0) * kSlotStride + f] = o[g][0];
-                    spec[(g * 4 + 1) * kSlotStride + f] = o[g][1];
+                    // into digit 0's row of either polynomial, which its warp owns
+                    spec[(g * 4 + 0) * kHalfN + ix] = o[g][0];
+                    spec[(g * 4 + 2) * kHalfN + ix] = o[g][1];
+                    if constexpr (KB) {
+                        const uint32_t a0 = rot[g], a1 = rot[g] >> 2;
+                        root[g][0] = mul_ipow(root[g][0], a0 + a1);
+                        root[g][1] = mul_ipow(root[g][1], a0);
+                        root[g][2] = mul_ipow(root[g][2], a1);
+                    }
                 }
             }
         }
         __syncthreads();
 
-        // ---- phase 3: inverse FFT + untwist + round, warp (g, j)
-        if (warp < 2 * G) {
-            const int g = warp >> 1, j = warp & 1;
-            double2* slot = spec + (g * 4 + j) * kSlotStride;
+        // ---- inverse transform of this warp's polynomial, rounding
+        {
             double2 v[16];
 #pragma unroll
-            for (int n2 = 0; n2 < 16; n2++) v[n2] = slot[lane + 32 * n2];
+            for (int k = 0; k < 16; k++) v[k] = slot[sl + 32 * k];
             __syncwarp();
-            ffnt_inverse_warp(v, slot, psi_s, lane);
-            uint32_t* a = acc + g * kTrlwe + j * kN;
+            tree16_inverse(v, slot, ltw, lane);
+            if constexpr (KB) {
+                const bool last = p + 1 == nsteps;
+                if (last) __syncthreads();  // the accumulators overwrite the spectra
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int n = ffnt_pos(lane, q);
-                // already untwisted and scaled to Torus32 units (x 2^23)
-                const double2 u = v[q];
-                const uint32_t lo = (uint32_t)__double2ll_rn(u.x);
-                const uint32_t hi = (uint32_t)__double2ll_rn(u.y);
-                if (KB) {
-                    a[acc_ix<KB>(n)] = lo;
-                    a[acc_ix<KB>(n + kHalfN)] = hi;
-                } else {
-                    a[n] += lo;
-                    a[n + kHalfN] += hi;
+                for (int q = 0; q < 16; q++) {
+                    const int m = tree_neg(q);
+                    const uint32_t lo = round_mod32(v[q].x) + recompose_lo(P[m]);
+                    const uint32_t hi = round_mod32(v[q].y) + recompose_hi(P[m]);
+                    P[m] = pack_halves(lo, hi);
+                    if (last) {
+                        own[low + 32 * m] = lo;
+                        own[low + 32 * m + 512] = hi;
+                    }
                 }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 16; q++) {
+                    const int n = low + 32 * tree_neg(q);
+                    own[n] += round_mod32(v[q].x);
+                    own[n + 512] += round_mod32(v[q].y);
+                }
+                __syncwarp();  // the next step's rotation reads other lanes' coefficients
             }
         }
-        __syncthreads();
     }
+    __syncthreads();
 
     // ---- epilogue: accumulator and/or SampleExtract (index 0)
     for (int g = 0; g < G; g++) {
         const int l = lane_base + g;
         if (l >= lanes) break;
-        const uint32_t* a = acc + g * kTrlwe;
+        const uint32_t* a = (KB ? reinterpret_cast<uint32_t*>(spec) : acc) + g * kTrlwe;
         if (acc_out)
-            for (int i = tid; i < kTrlwe; i += blockDim.x)
-                acc_out[(size_t)l * kTrlwe + i] = a[acc_ix<KB>(i)];
+            for (int i = tid; i < kTrlwe; i += NT) acc_out[(size_t)l * kTrlwe + i] = a[i];
         if (lane_out) {
             uint32_t* o = lane_out + (size_t)l * kTlwe1;
-            for (int i = tid; i <= kN; i += blockDim.x)
-                o[i] = i == kN ? a[acc_ix<KB>(kN)] : (i == 0 ? a[0] : 0u - a[acc_ix<KB>(kN - i)]);
+            for (int i = tid; i <= kN; i += NT)
+                o[i] = i == kN ? a[kN] : (i == 0 ? a[0] : 0u - a[kN - i]);
         }
     }
+}
+
+template <bool KB, int MINB>
+cudaError_t launch_two(const uint32_t* lane_in, int lanes, uint32_t mu, const double2* bkf,
+                       const Fp64Tables& t, int steps, uint32_t* acc_out, uint32_t* lane_out,
+                       cudaStream_t st)
+{
+    constexpr size_t smem = two_smem_bytes<KB>();
+    static DeviceAttrFlags attr;
+    {
+        const cudaError_t e = set_smem_attr_once(attr, k_br_fp64<KB, MINB>, smem);
+        if (e != cudaSuccess) return e;
+    }
+    k_br_fp64<KB, MINB><<<(lanes + 1) / 2, 128, smem, st>>>(lane_in, lanes, mu, bkf, t.psi, steps,
+                                                          acc_out, lane_out);
+    return cudaGetLastError();
 }
 
 // BK polynomial -> Fourier domain: read as signed int32, scale 2^-32, fold,
@@ -314,7 +344,7 @@ __global__ void __launch_bounds__(G * 128, G == 1 ? 3 : (G == 2 ? 2 : 1)) k_br_f
 __global__ void __launch_bounds__(128) k_bk_to_fft(const uint32_t* __restrict__ bk, int npolys,
                                                    const double2* __restrict__ psi,
                                                    const double2* __restrict__ tw512,
-                                                   double2* __restrict__ out)
+                                                   double2* __restrict__ out, int pairs)
 {
     __shared__ __align__(16) double2 tiles[4][kSlotStride];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -330,242 +360,251 @@ __global__ void __launch_bounds__(128) k_bk_to_fft(const uint32_t* __restrict__ 
         v[n2] = cmul(z, __ldg(&psi[n]));
     }
     fft512_warp<1>(v, tiles[warp], tw512, lane);
-    double2* dst = out + (size_t)poly * kHalfN;
+    // pairs: bins of the two polynomials of a row interleaved
+    double2* dst = pairs ? out + (size_t)(poly >> 1) * 2 * kHalfN + (poly & 1)
+                         : out + (size_t)poly * kHalfN;
+    const int step = pairs ? 2 : 1;
 #pragma unroll
-    for (int m = 0; m < 16; m++) dst[(lane & 15) + 16 * m + 256 * (lane >> 4)] = v[m];
+    for (int m = 0; m < 16; m++) dst[step * ((lane & 15) + 16 * m + 256 * (lane >> 4))] = v[m];
 }
 
-template <bool KB, int G>
-cudaError_t launch_g(const uint32_t* lane_in, int lanes, uint32_t mu, const double2* bkf,
-                     const Fp64Tables& t, int steps, uint32_t* acc_out, uint32_t* lane_out,
-                     cudaStream_t st)
+// ---- one lane per CTA (R = 1), or per cluster of R = 4 CTAs on 4 SMs; two warps per
+// digit row (8 points per thread), since a warp alone cannot keep the FP64 pipe
+// busy.  In a cluster every CTA runs the lane's transforms (redundantly, on its
+// own copy of the accumulator) but multiplies only its 512 / R frequency bins
+// with the key, and the inverse transforms gather the parts from the peers'
+// shared memory (distributed shared memory).  The key rows of a step do not
+// depend on the step before, so each thread fetches those of its first items
+// into registers before the forward transforms and those of a further one while
+// it multiplies, and the rows of the step after next are brought into the L2:
+// a gate's key switching key and this key together do not stay there (32 lanes
+// between key switches: one CTA per lane without the prefetch 2.30 ms, with it
+// 1.25, in clusters 1.05; nothing else between the rotations 1.6 ms).  The products of a cluster alternate
+// between two buffers, so that one cluster barrier per step is enough: a buffer
+// is rewritten two steps later, after the next step's barrier, which every
+// peer's gather precedes.
+// One lane: 1.22 -> 1.06 ms (R = 4); 148 lanes 1.66 -> 1.15 (R = 1); 296 lanes,
+// two CTAs per SM, 2.18 -> 1.95; 444 lanes, three, 2.95 -> 2.75.  Plain key:
+// 148 lanes 2.71 -> 1.71, 296 lanes 3.44 -> 2.88, 444 lanes 4.56 -> 4.18 ms.
+// Measured and not kept: clusters of two up to 74 lanes (no gain over one CTA;
+// plain key 2.06 against 1.67 ms), neighbouring threads sharing a bin with one
+// output each (148 lanes 1.21 ms), the twiddles in shared memory (1.17-1.21 ms).
+constexpr int kCluMaxLanes = 32;
+constexpr size_t kOneSmem = 120 * 1024;  // > half an SM: one CTA per SM
+template <int R>
+constexpr size_t one_smem_bytes()
 {
-    constexpr size_t smem = br_smem_bytes<G>();
-    static DeviceAttrFlags attr;
-    {
-        const cudaError_t e = set_smem_attr_once(attr, k_br_fp64<KB, G>, smem);
-        if (e != cudaSuccess) return e;
-    }
-    const int blocks = (lanes + G - 1) / G;
-    k_br_fp64<KB, G><<<blocks, G * 128, smem, st>>>(lane_in, lanes, mu, bkf, t.psi, t.tw512, steps,
-                                                    acc_out, lane_out);
-    return cudaGetLastError();
+    return sizeof(double2) * ((R > 1 ? 8 : 4) * kHalfN + kRootEntries) + sizeof(uint32_t) * kTrlwe +
+           sizeof(uint16_t) * kN0;
+}
+static_assert(one_smem_bytes<4>() <= kOneSmem && one_smem_bytes<1>() <= 75 * 1024, "CTA layouts");
+
+// the key words of both output polynomials of a row, fetched where the program
+// says so (volatile: not moved down to their use, past the transforms or a
+// barrier)
+__device__ __forceinline__ void key_words(double2 (&k)[2], const double2* p)
+{
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(k[0].x), "=d"(k[0].y), "=d"(k[1].x), "=d"(k[1].y) : "l"(p));
 }
 
-// ---- latency form for small batches: one lane per cluster of four CTAs on
-// four SMs.  A single lane's step is bound by the rate at which one SM pulls
-// the step's key rows from L2 (196 KB per KeyBundle step); here every CTA of
-// the cluster runs the lane's transforms (redundantly, on its own copy of the
-// accumulator) but multiplies only its quarter of the frequency bins with the
-// key, and the inverse transforms gather the four quarters from the peers'
-// shared memory (distributed shared memory).  The arithmetic of every bin is
-// that of k_br_fp64, so the result is bit-identical.
-constexpr int kCluRanks = 4;
-constexpr int kCluMaxLanes = 16;         // measured: faster than one CTA per lane up to 16 lanes
-constexpr size_t kCluSmem = 120 * 1024;  // > half an SM: one CTA per SM
-
-template <bool KB>
-__global__ void __cluster_dims__(kCluRanks, 1, 1) __launch_bounds__(128, 1)
-    k_br_fp64_clu(const uint32_t* __restrict__ lane_in, int lanes, uint32_t mu,
+template <bool KB, int R, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+    k_br_fp64_one(const uint32_t* __restrict__ lane_in, int lanes, uint32_t mu,
                   const double2* __restrict__ bkf, const double2* __restrict__ psi, int steps,
                   uint32_t* __restrict__ acc_out, uint32_t* __restrict__ lane_out)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char smem[];
-    double2* spec = reinterpret_cast<double2*>(smem);
-    double2* psi_s = spec + 4 * kSlotStride;
-    uint32_t* acc = reinterpret_cast<uint32_t*>(psi_s + kN);
+    double2* spec = reinterpret_cast<double2*>(smem);  // [4][512] digit spectra
+    // [2][2][512] products, by step parity; one CTA: in the place of rows 0 and 2
+    double2* prod = R > 1 ? spec + 4 * kHalfN : spec;
+    double2* roots = R > 1 ? prod + 4 * kHalfN : spec + 4 * kHalfN;
+    uint32_t* acc = reinterpret_cast<uint32_t*>(roots + kRootEntries);
     uint16_t* abar = reinterpret_cast<uint16_t*>(acc + kTrlwe);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int rank = (int)cluster.block_rank();
-    const int l = blockIdx.x / kCluRanks;
+    const int tid = threadIdx.x;
+    const int pair = tid >> 6, T = tid & 63, bar_id = 1 + pair;
+    const int rank = R > 1 ? (int)cluster.block_rank() : 0;
+    const double2* const ltw = psi + 2 * kN + T;
+    const int l = blockIdx.x / R;
     const bool ok = l < lanes;
 
-    for (int t = tid; t < kN; t += blockDim.x) psi_s[psi_pos((uint32_t)t)] = psi[t];
+    for (int t = tid; t <= 512; t += 256) roots[root_pos((uint32_t)t)] = psi[t];
     {
         const uint32_t* x = lane_in + (size_t)(ok ? l : 0) * kTlwe0;
-        for (int i = tid; i < kN0; i += blockDim.x)
-            abar[i] = ok ? (uint16_t)((x[i] + (1u << 20)) >> 21) : 0;
+        for (int i = tid; i < kN0; i += 256) abar[i] = ok ? (uint16_t)((x[i] + (1u << 20)) >> 21) : 0;
         const uint32_t bar = ok ? 2u * kN - (x[kN0] >> 21) : 2u * kN;
-        for (int i = tid; i < kN; i += blockDim.x) {
+        for (int i = tid; i < kN; i += 256) {
             acc[i] = 0;
-            uint32_t v;
-            if (bar == 2u * kN)
-                v = mu;
-            else
-                v = (((uint32_t)i < (bar & (kN - 1))) ^ (bar >> 10)) ? 0u - mu : mu;
-            acc[kN + i] = v;
+            acc[kN + i] = test_coef(bar, (uint32_t)i, mu);
         }
     }
-    // the peers' transform slots 0 and 1 (the multiply-accumulate results)
-    const double2* peer[kCluRanks];
+    const double2* peer[R];
 #pragma unroll
-    for (int k = 0; k < kCluRanks; k++) peer[k] = cluster.map_shared_rank(spec, k);
-    cluster.sync();
+    for (int k = 0; k < R; k++) peer[k] = R > 1 ? cluster.map_shared_rank(prod, k) : prod;
+    if (R > 1) cluster.sync(); else __syncthreads();
 
     const int total = KB ? kN0 / 2 : kN0;
     const int nsteps = (steps < 0 || steps > total) ? total : steps;
+    constexpr int E = KB ? 3 : 1;                    // keys per step
+    constexpr int NB = R == 1 ? 2 : 1;               // bins per thread
     constexpr size_t kTrgswF = 4 * 2 * kHalfN;
+    const int f0 = rank * (512 / R) + tid;
+    const bool mac = R < 4 || tid < 512 / R;
 
 #pragma unroll 1
     for (int p = 0; p < nsteps; p++) {
-        // ---- phase 1 (every rank): decompose + fold + twist + forward FFT, warp r
+        if (tid == 0 && p + 2 < nsteps)
+            prefetch_part(bkf + (size_t)(p + 2) * E * kTrgswF, E * kTrgswF * sizeof(double2), blockIdx.x,
+                          gridDim.x);
+        const double2* bk = bkf + (size_t)p * E * kTrgswF + 2 * f0;
+        constexpr int NPRE = MINB > 2 ? 0 : MINB > 1 ? 1 : E;  // keys fetched ahead
+        double2 b[E][4][2];
+        if (mac)
+#pragma unroll
+            for (int e = 0; e < NPRE; e++)
+#pragma unroll
+                for (int r = 0; r < 4; r++) key_words(b[e][r], &bk[(e * 4 + r) * 1024]);
+        // ---- phase 1 (every rank): decompose + fold + forward transform, pair r
         {
-            const int r = warp, j = r >> 1, d = r & 1;
-            const uint32_t* a = acc + j * kN;
-            double2 v[16];
+            const int d = pair & 1;
+            const uint32_t* a = acc + (pair >> 1) * kN;
+            double2 v[8];
             const uint32_t ab = KB ? 0u : abar[p];
             const uint32_t abm = ab & (kN - 1), abn = ab >> 10;
 #pragma unroll
-            for (int n2 = 0; n2 < 16; n2++) {
-                const int n = lane + 32 * n2;
-                uint32_t lo = a[n], hi = a[n + kHalfN];
-                if (!KB) {
-                    uint32_t rl = a[(n - ab) & (kN - 1)];
-                    uint32_t rh = a[(n + kHalfN - ab) & (kN - 1)];
-                    rl = (((uint32_t)n < abm) ^ abn) ? 0u - rl : rl;
-                    rh = (((uint32_t)(n + kHalfN) < abm) ^ abn) ? 0u - rh : rh;
+            for (int m = 0; m < 8; m++) {
+                const uint32_t n = (uint32_t)(T + 64 * m);
+                uint32_t lo = a[n], hi = a[n + 512];
+                if constexpr (!KB) {
+                    uint32_t rl = a[(n - ab) & (kN - 1)], rh = a[(n + 512 - ab) & (kN - 1)];
+                    rl = ((n < abm) ^ abn) ? 0u - rl : rl;
+                    rh = ((n + 512 < abm) ^ abn) ? 0u - rh : rh;
                     lo = rl - lo;
                     hi = rh - hi;
                 }
-                v[n2] = make_double2(digit_of(lo + kDecOffset, d), digit_of(hi + kDecOffset, d));
+                v[m] = digits_of(pack_halves(lo, hi), d);
             }
-            double2* slot = spec + r * kSlotStride;
-            ffnt_forward_warp(v, slot, psi_s, lane);
-#pragma unroll
-            for (int q = 0; q < 16; q++) slot[ffnt_pos(lane, q)] = v[q];
+            tree_forward(v, spec + pair * kHalfN, ltw, T, bar_id);
+            tree_store(v, spec + pair * kHalfN, T);
         }
         __syncthreads();
 
-        // ---- phase 2 (rank k): key multiply-accumulate of bins [128 k, 128 k + 128)
-        {
-            const int f = rank * 128 + tid;
-            double2 D[4];
+        // ---- phase 2: key multiply-accumulate of this rank's bins
+        if (mac)
 #pragma unroll
-            for (int r = 0; r < 4; r++) D[r] = spec[r * kSlotStride + f];
-            double2 out0;
-            if (KB) {
-                const double2* bk = bkf + (size_t)p * 3 * kTrgswF;
+            for (int u = 0; u < NB; u++) {
+                const int f = f0 + 256 * u;
+                const int ix = spec_ix(f);
+                double2 D[4], o[2];
+                o[0] = o[1] = make_double2(0.0, 0.0);
+#pragma unroll
+                for (int r = 0; r < 4; r++) D[r] = spec[r * kHalfN + ix];
                 const uint32_t ef = 1u + 4u * (uint32_t)f;
-                const uint32_t a0 = abar[2 * p], a1 = abar[2 * p + 1];
-                double2 x0 = psi_at(psi_s, ef * a0);
-                double2 x1 = psi_at(psi_s, ef * a1);
-                double2 x01 = psi_at(psi_s, ef * (a0 + a1));
-                x0.x -= 1.0;
-                x1.x -= 1.0;
-                x01.x -= 1.0;
+                const uint32_t a0 = abar[KB ? 2 * p : 0], a1 = abar[KB ? 2 * p + 1 : 0];
+                const uint32_t am[3] = {a0 + a1, a0, a1};
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    double2 b[3][4];
+                for (int e = 0; e < E; e++) {
+                    if (u == 0 && e >= NPRE)
 #pragma unroll
-                    for (int e = 0; e < 3; e++)
-#pragma unroll
-                        for (int r = 0; r < 4; r++)
-                            b[e][r] = __ldg(&bk[((e * 4 + r) * 2 + j) * kHalfN + f]);
-                    double2 s0 = make_double2(0.0, 0.0), s1 = s0, s2 = s0;
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        s0 = cfma(s0, D[r], b[0][r]);
-                        s1 = cfma(s1, D[r], b[1][r]);
-                        s2 = cfma(s2, D[r], b[2][r]);
-                    }
-                    double2 o = make_double2(fma(D[2 * j].x, 0x1p-8, D[2 * j + 1].x * 0x1p-16),
-                                             fma(D[2 * j].y, 0x1p-8, D[2 * j + 1].y * 0x1p-16));
-                    o = cfma(o, x01, s0);
-                    o = cfma(o, x0, s1);
-                    o = cfma(o, x1, s2);
-                    if (j == 0)
-                        out0 = o;
-                    else {
-                        spec[0 * kSlotStride + f] = out0;
-                        spec[1 * kSlotStride + f] = o;
-                    }
-                }
-            } else {
-                const double2* bk = bkf + (size_t)p * kTrgswF;
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    double2 o = make_double2(0.0, 0.0);
+                        for (int r = 0; r < 4; r++) key_words(b[e][r], &bk[(e * 4 + r) * 1024]);
+                    double2 s[2];
 #pragma unroll
                     for (int r = 0; r < 4; r++)
-                        o = cfma(o, D[r], __ldg(&bk[(r * 2 + j) * kHalfN + f]));
-                    if (j == 0)
-                        out0 = o;
-                    else {
-                        spec[0 * kSlotStride + f] = out0;
-                        spec[1 * kSlotStride + f] = o;
+#pragma unroll
+                        for (int j = 0; j < 2; j++)
+                            s[j] = cfma(r ? s[j] : make_double2(0.0, 0.0), D[r], b[e][r][j]);
+                    if (u + 1 < NB)
+#pragma unroll
+                        for (int r = 0; r < 4; r++) key_words(b[e][r], &bk[(e * 4 + r) * 1024 + 512]);
+                    if constexpr (KB) {
+                        // sum of (X^a - 1) bk terms; H is added as an integer (phase 3)
+                        double2 x = root_at(roots, ef * am[e]);
+                        x.x -= 1.0;
+                        o[0] = cfma(o[0], x, s[0]);
+                        o[1] = cfma(o[1], x, s[1]);
+                    } else {
+                        o[0] = s[0];
+                        o[1] = s[1];
                     }
                 }
+                double2* const out = R > 1 ? prod + (p & 1) * 2 * kHalfN : spec;
+                out[ix] = o[0];
+                out[(R > 1 ? 1 : 2) * kHalfN + ix] = o[1];
             }
-        }
-        cluster.sync();  // every rank's quarter of slots 0 and 1 is written
+        if (R > 1) cluster.sync(); else __syncthreads();  // every rank's products are written
 
-        // ---- phase 3 (every rank): gather, inverse FFT, untwist, round, warp j
-        if (warp < 2) {
-            const int j = warp;
-            double2 v[16];
+        // ---- phase 3 (every rank): gather, inverse transform, round, pair j
+        if (pair < 2) {
+            const int f = spec_ix(tree_bin(T));
+            double2 v[8];
 #pragma unroll
-            for (int n2 = 0; n2 < 16; n2++)
-                v[n2] = peer[n2 >> 2][j * kSlotStride + lane + 32 * n2];
-            double2* scratch = spec + (2 + j) * kSlotStride;  // rows 2, 3 are free now
-            ffnt_inverse_warp(v, scratch, psi_s, lane);
-            uint32_t* a = acc + j * kN;
+            for (int k = 0; k < 8; k++) 
+                v[k] = R > 1 ? peer[k * R / 8][((p & 1) * 2 + pair) * kHalfN + f + 64 * k]
+                             : spec[2 * pair * kHalfN + f + 64 * k];
+            tree_inverse(v, spec + 2 * pair * kHalfN, ltw, T, bar_id);
+            uint32_t* a = acc + pair * kN;
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                const int n = ffnt_pos(lane, q);
-                const double2 u = v[q];  // untwisted, in Torus32 units
-                const uint32_t lo = (uint32_t)__double2ll_rn(u.x);
-                const uint32_t hi = (uint32_t)__double2ll_rn(u.y);
-                if (KB) {
-                    a[n] = lo;
-                    a[n + kHalfN] = hi;
-                } else {
-                    a[n] += lo;
-                    a[n + kHalfN] += hi;
-                }
+            for (int q = 0; q < 8; q++) {
+                const int n = T + 64 * neg8(q);
+                const uint32_t lo = round_mod32(v[q].x), hi = round_mod32(v[q].y);
+                a[n] = lo + (KB ? (a[n] + (1u << 15)) & 0xffff0000u : a[n]);
+                a[n + 512] = hi + (KB ? (a[n + 512] + (1u << 15)) & 0xffff0000u : a[n + 512]);
             }
         }
-        cluster.sync();  // the gathers are done before slots 0 and 1 are rewritten
+        __syncthreads();
     }
+    if (R > 1) cluster.sync();  // no CTA leaves while a peer still gathers from it
 
     if (ok && rank == 0) {
         if (acc_out)
-            for (int i = tid; i < kTrlwe; i += blockDim.x) acc_out[(size_t)l * kTrlwe + i] = acc[i];
+            for (int i = tid; i < kTrlwe; i += 256) acc_out[(size_t)l * kTrlwe + i] = acc[i];
         if (lane_out) {
             uint32_t* o = lane_out + (size_t)l * kTlwe1;
-            for (int i = tid; i <= kN; i += blockDim.x)
+            for (int i = tid; i <= kN; i += 256)
                 o[i] = i == kN ? acc[kN] : (i == 0 ? acc[0] : 0u - acc[kN - i]);
         }
     }
 }
 
-template <bool KB>
-cudaError_t launch_clu(const uint32_t* lane_in, int lanes, uint32_t mu, const double2* bkf,
+template <bool KB, int R, int MINB>
+cudaError_t launch_one(const uint32_t* lane_in, int lanes, uint32_t mu, const double2* bkf,
                        const Fp64Tables& t, int steps, uint32_t* acc_out, uint32_t* lane_out,
                        cudaStream_t st)
 {
     static DeviceAttrFlags attr;
+    constexpr size_t smem = MINB == 1 ? kOneSmem : one_smem_bytes<R>();
     {
-        const cudaError_t e = set_smem_attr_once(attr, k_br_fp64_clu<KB>, kCluSmem);
+        const cudaError_t e = set_smem_attr_once(attr, k_br_fp64_one<KB, R, MINB>, smem);
         if (e != cudaSuccess) return e;
     }
-    k_br_fp64_clu<KB><<<lanes * kCluRanks, 128, kCluSmem, st>>>(lane_in, lanes, mu, bkf, t.psi, steps,
-                                                              acc_out, lane_out);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(lanes * R);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = R;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = R > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_br_fp64_one<KB, R, MINB>, lane_in, lanes, mu, bkf, t.psi, steps,
+                              acc_out, lane_out);
 }
 }  // namespace
 
-// Lanes per CTA: 1 (three CTAs per SM), 2 (two CTAs per SM, whose phases
-// overlap) or 4 (one CTA per SM, key rows shared by 4 lanes).  CUFHE_BR_LANES_PER_CTA overrides the
-// default for tuning.
+// Lanes per CTA: 1 or 2 (4, an earlier form, is taken as 2).
+// CUFHE_BR_LANES_PER_CTA overrides the default for tuning.
 static int br_lanes_per_cta()
 {
     static int g = 0;
     if (!g) {
         const char* e = getenv("CUFHE_BR_LANES_PER_CTA");
-        g = (e && atoi(e) == 4) ? 4 : (e && atoi(e) == 2) ? 2 : (e && atoi(e) == 1) ? 1 : kDefaultBrGates;
+        g = (e && atoi(e) == 4) ? 4 : (e && atoi(e) == 2) ? 2 : (e && atoi(e) == 1) ? 1 : 2;
     }
     return g;
 }
@@ -615,10 +654,11 @@ cudaError_t launch_br_fp64(bool kb, const uint32_t* lane_in, int lanes, uint32_t
         while (i + 1 < tun.n && lanes > tun.bound[i]) i++;
         g = tun.g[i];
     } else {
-        // untuned: one lane per CTA (3 CTAs per SM) while the batch fits one
-        // wave, which minimises latency; larger ones: two lanes per CTA
+        // untuned: one lane per CTA while the batch fits one round of three
+        // per SM (444 lanes: 2.75 ms against 3.2 ms with two lanes per CTA),
+        // two lanes per CTA beyond (592 lanes: 3.18 against 3.9 ms)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        g = lanes <= 3 * sms ? 1 : kDefaultBrGates;
+        g = lanes <= 3 * sms ? 1 : 2;
     }
     return launch_br_fp64_g(g, kb, lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st);
 }
@@ -628,55 +668,57 @@ cudaError_t launch_br_fp64_g(int g, bool kb, const uint32_t* lane_in, int lanes,
                              uint32_t* acc_out, uint32_t* lane_out, cudaStream_t st)
 {
     if (lanes <= 0) return cudaSuccess;
-    if (g == 1 && lanes <= kCluMaxLanes) {
-        // small batches: one lane per cluster of four SMs (CUFHE_BR_CLUSTER=0
-        // keeps one CTA per lane); a device that cannot place the clusters
-        // runs the one-CTA kernel instead
-        int sms = 148, dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const char* e = getenv("CUFHE_BR_CLUSTER");
-        if (lanes * kCluRanks <= sms && !(e && atoi(e) == 0)) {
-            const cudaError_t r =
-                kb ? launch_clu<true>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st)
-                   : launch_clu<false>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st);
-            if (r == cudaSuccess) return r;
-            cudaGetLastError();
-        }
+    int sms = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+#define BR_ARGS lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st
+    if (g != 1) {
+        // plain: shared memory for two CTAs per SM.  KeyBundle: two when that
+        // is one round (4 lanes per SM), three beyond.
+        if (!kb) return launch_two<false, 2>(BR_ARGS);
+        return lanes <= 4 * sms ? launch_two<true, 2>(BR_ARGS) : launch_two<true, 3>(BR_ARGS);
     }
-    if (g == 1)
-        return kb ? launch_g<true, 1>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st)
-                  : launch_g<false, 1>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st);
-    if (g == 2)
-        return kb ? launch_g<true, 2>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st)
-                  : launch_g<false, 2>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st);
-    return kb ? launch_g<true, 4>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st)
-              : launch_g<false, 4>(lane_in, lanes, mu, bkf, t, steps, acc_out, lane_out, st);
+    // KeyBundle: one lane per cluster of four SMs while the clusters fit at once
+    // (32 lanes: 1.05 against 1.14 ms; 37 clusters no longer fit: 2.2 ms).  The
+    // plain key has a third of the key rows per step and gains nothing (one lane
+    // 2.03 against 1.64 ms).  CUFHE_BR_CLUSTER=0 keeps one CTA per lane; a device
+    // that cannot place the clusters runs one CTA per lane instead.
+    const char* e = getenv("CUFHE_BR_CLUSTER");
+    if (kb && !(e && atoi(e) == 0) && lanes <= kCluMaxLanes && 4 * lanes <= sms) {
+        const cudaError_t r = launch_one<true, 4, 1>(BR_ARGS);
+        if (r == cudaSuccess) return r;
+        cudaGetLastError();
+    }
+    if (lanes <= sms) return kb ? launch_one<true, 1, 1>(BR_ARGS) : launch_one<false, 1, 1>(BR_ARGS);
+    if (lanes <= 2 * sms) return kb ? launch_one<true, 1, 2>(BR_ARGS) : launch_one<false, 1, 2>(BR_ARGS);
+    return kb ? launch_one<true, 1, 3>(BR_ARGS) : launch_one<false, 1, 3>(BR_ARGS);
+#undef BR_ARGS
 }
 
 cudaError_t launch_bk_to_fft(const uint32_t* bk, int npolys, const Fp64Tables& t, double2* out,
-                             cudaStream_t st)
+                             cudaStream_t st, bool pairs)
 {
-    k_bk_to_fft<<<(npolys + 3) / 4, 128, 0, st>>>(bk, npolys, t.psi, t.tw512, out);
+    k_bk_to_fft<<<(npolys + 3) / 4, 128, 0, st>>>(bk, npolys, t.psi, t.tw512, out, pairs ? 1 : 0);
     return cudaGetLastError();
 }
 
 cudaError_t upload_fft_constants(void)
 {
-    double2 w[16], t32[16], uq[16];
+    double2 w[16], un[8];
     const long double pi = 3.141592653589793238462643383279502884L;
     for (int k = 0; k < 16; k++) {
         const long double a = 2 * pi * k / 32;
         w[k] = make_double2((double)cosl(a), (double)sinl(a));
-        const long double b = pi * k / 32;  // psi^{32 k}
-        t32[k] = make_double2((double)cosl(b), (double)sinl(b));
-        // conj(psi^{16 (k mod 8) + 256 (k / 8)}) 2^23
-        const long double c = -pi * (16 * (k & 7) + 256 * (k >> 3)) / 1024;
-        uq[k] = make_double2((double)(cosl(c) * 0x1p23L), (double)(sinl(c) * 0x1p23L));
     }
+    for (int k = 0; k < 8; k++) {
+        const long double b = -pi * k / 16;  // psi^{-64 k}, times 2^23
+        un[k] = make_double2((double)(cosl(b) * 0x1p23L), (double)(sinl(b) * 0x1p23L));
+    }
+    double2 un16[16];
+    untwist16(un16);
     cudaError_t e = cudaMemcpyToSymbol(c_w32, w, sizeof(w));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_tw32, t32, sizeof(t32));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_utwq, uq, sizeof(uq));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_untw, un, sizeof(un));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_untw16, un16, sizeof(un16));
     return e;
 }
 

@@ -249,11 +249,27 @@ cufhe_stream_s* resolve(cufhe_stream_t st)
 void host_tables(std::vector<double2>& psi, std::vector<double2>& tw)
 {
     const long double pi = 3.141592653589793238462643383279502884L;
-    psi.resize(2 * kN);
+    psi.resize(kTw16At + kLaneTw16 * 32);
     for (int t = 0; t < 2 * kN; t++) {
         const long double a = pi * t / kN;  // psi = e^{i pi / N}
         psi[t] = make_double2((double)cosl(a), (double)sinl(a));
     }
+    for (int e = 0; e < kLaneTw; e++)
+        for (int T = 0; T < 64; T++) {
+            const int w = T & 7, r = T >> 3, f = r + 8 * w;
+            const int t = e < 3   ? (1 + 4 * r) << (5 - e)
+                          : e < 6 ? (1 + 4 * f) << (5 - e)
+                          : e < 9 ? -w * (1 << (13 - e))
+                                  : -T * (e < 12 ? 1 << (13 - e) : 1);
+            psi[2 * kN + e * 64 + T] = psi[t & (2 * kN - 1)];
+        }
+    for (int e = 0; e < kLaneTw16; e++)
+        for (int l = 0; l < 32; l++) {
+            const int c = (l >> 1) + 16 * (l & 1);
+            const int t = e < 5 ? (1 + 4 * c) << (4 - e)
+                                : -c * (e < 9 ? 4 << (8 - e) : e == 9 ? 64 : 1);
+            psi[kTw16At + e * 32 + l] = psi[t & (2 * kN - 1)];
+        }
     tw.resize(16 * 32);
     for (int k2 = 0; k2 < 16; k2++)
         for (int n1 = 0; n1 < 32; n1++) {
@@ -338,7 +354,7 @@ int init_device(int d, const cufhe_keyview* ek)
     const int npolys = (int)(ek->bk_words / kN);
     CK(cudaMalloc(&D.bkf, (size_t)npolys * 512 * sizeof(double2)));
     const Fp64Tables t = {D.psi, D.tw512};
-    CKL(launch_bk_to_fft(raw, npolys, t, D.bkf, 0));
+    CKL(launch_bk_to_fft(raw, npolys, t, D.bkf, 0, true));
     {
         // INT8 Toeplitz limb windows of either key form (KeyBundle: 954 TRGSWs)
         cudaError_t e = int8_key_build(D.i8, raw, ek->keybundle != 0, 0);
@@ -2266,7 +2282,7 @@ int cufhe_trgsw_to_fft(int gadget, const uint32_t* trgsw, size_t count, double* 
     const Fp64Tables t = {psi, tw};
     LAUNCH(CUFHE_K_CMUX, s->st,
            launch_bk_to_fft(trgsw, (int)(count * 2 * gadget_rows(gadget)), t,
-                            reinterpret_cast<double2*>(fft_out), s->st));
+                            reinterpret_cast<double2*>(fft_out), s->st, false));
     return CUFHE_OK;
 }
 

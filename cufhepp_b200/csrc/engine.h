@@ -208,16 +208,30 @@ cudaError_t launch_copy_rows(const int32_t* rows, int nrows, int words, const ui
 // FP64 FFNT blind rotation + SampleExtract of `lanes` lvl0 TLWEs.
 // acc_out (optional) receives the TRLWE accumulators; lane_out (optional) the
 // extracted lvl1 TLWEs.  steps < 0: all steps.
+// Twiddles of the transforms (ffnt_tree.cuh), behind the root table:
+// [kLaneTw][64], one column per thread T (w = T mod 8, r = T div 8, f = r + 8 w).
+// Forward passes: psi^{(1 + 4 r) 2^{5 - e}} (e = 0..2), psi^{(1 + 4 f) 2^{5 - e}}
+// (e = 3..5); inverse passes: psi^{-w 2^{13 - e}} (e = 6..8), psi^{-T 2^{13 - e}}
+// (e = 9..11), psi^{-T} (e = 12).
+// Behind them the twiddles of the one-warp transforms (ffnt_tree16.cuh),
+// [kLaneTw16][32], l = lane div 2 + 16 (lane mod 2): psi^{(1 + 4 l) 2^{4 - e}}
+// (e = 0..4), psi^{-l 2^{10 - e}} (e = 5..8), psi^{-64 l} (e = 9), psi^{-l}
+// (e = 10).
+constexpr int kLaneTw = 13, kLaneTw16 = 11;
+constexpr int kTw16At = 2 * CUFHE_LVL1_N + kLaneTw * 64;  // where the latter begin
 struct Fp64Tables {
-    const double2* psi;    // psi^t, t < 2048, psi = e^{i pi / 1024}
+    const double2* psi;    // psi^t, t < 2048, psi = e^{i pi / 1024}; then the lane twiddles
     const double2* tw512;  // [16][32] e^{2 pi i n1 k2 / 512}
 };
 cudaError_t launch_br_fp64(bool kb, const uint32_t* lane_in, int lanes, uint32_t mu,
                            const double2* bkf, const Fp64Tables& t, int steps,
                            uint32_t* acc_out, uint32_t* lane_out, cudaStream_t st);
 
+// Fourier form of npolys polynomials, natural bin order; pairs: bins of
+// polynomials 2 i and 2 i + 1 (a key row's two) interleaved, as the blind
+// rotation reads them
 cudaError_t launch_bk_to_fft(const uint32_t* bk, int npolys, const Fp64Tables& t, double2* out,
-                             cudaStream_t st);
+                             cudaStream_t st, bool pairs);
 // The same rotation with a fixed number of lanes per CTA (1, 2 or 4), for the
 // autotuner; launch_br_fp64 picks it from the tuned table of the device
 // (br_fp64_set_tuning) or, without one, from the batch size.

@@ -14,10 +14,10 @@
 //      DFT over m in registers.
 //   5. one radix-2 stage across lanes l and l ^ 16 (warp shuffle).
 //   Output: lane (k2 + 16 h), register m holds bin k2 + 16 m + 256 h
-//   (fft512_warp: key conversion, CMUX).  The blind-rotation transforms
-//   (ffnt_forward_warp / ffnt_inverse_warp and the N = 2048 halves) run step
-//   5 with both lanes of a pair busy (radix2_pair) and leave register q at
-//   ffnt_pos(lane, q) instead.
+//   (fft512_warp: key conversion, CMUX).  The halves of the N = 2048 transforms
+//   run step 5 with both lanes of a pair busy (radix2_pair) and leave register
+//   q at ffnt_pos(lane, q) instead.  The N = 1024 blind rotations have
+//   transforms of their own (ffnt_tree.cuh, ffnt_tree16.cuh).
 //
 // The reference runs one 512-point FFT per CTA with 256 threads and
 // __syncthreads between stages; here a warp owns a whole transform and only
@@ -31,6 +31,25 @@ namespace cufhe {
 
 constexpr int kHalfN = 512;
 constexpr int kSlotStride = 528;  // double2 per transform slot (16 x 33 tile)
+
+// the key words of both output polynomials of a row, side by side
+__device__ __forceinline__ void key_pair(double2& k0, double2& k1, const double2* p)
+{
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(k0.x), "=d"(k0.y), "=d"(k1.x), "=d"(k1.y) : "l"(p));
+}
+
+// Key rows of a later step into L2 (the key shares the L2 with the rest of a
+// gate's data): CTA i of n fetches the i-th part of `bytes`
+__device__ __forceinline__ void prefetch_part(const void* p, uint32_t bytes, uint32_t i, uint32_t n)
+{
+    const uint32_t part = ((bytes / n + 127u) & ~127u);
+    const uint32_t at = part * i;
+    if (at >= bytes) return;
+    const uint32_t len = bytes - at < part ? bytes - at : part;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                 ::"l"(reinterpret_cast<const char*>(p) + at), "r"(len) : "memory");
+}
 
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
@@ -168,35 +187,14 @@ __device__ __forceinline__ void fft512_warp(double2 (&v)[16], double2* tile,
     }
 }
 
-// ---------------------------------------------------------------------------
-// Transforms of the lvl1 blind-rotation kernels.  The root table psi^t
-// (t < N, psi = e^{i pi / N}; psi^{t+N} = -psi^t) lives in shared memory in
-// the interleaved order pos(t) = (t mod 4) * 256 + t / 4, which makes the
-// KeyBundle gathers psi^{(1+4f) a} (stride 4a across lanes) bank-conflict
-// free for odd a.
-__device__ __forceinline__ int psi_pos(uint32_t t) { return (int)((t & 3u) * 256u + ((t >> 2) & 255u)); }
-
-// psi^t for any t (mod 2N)
-__device__ __forceinline__ double2 psi_at(const double2* psi_s, uint32_t t)
-{
-    double2 v = psi_s[psi_pos(t)];
-    if (t & 1024u) {
-        v.x = -v.x;
-        v.y = -v.y;
-    }
-    return v;
-}
-
-// e^{i pi n2 / 32} (= psi^{32 n2}, the compile-time part of the forward
-// twist) and c_utwq[q] = e^{-i pi ((q mod 8) + 16 (q / 8)) / 64} times a
-// power of two that each translation unit chooses (the compile-time part of
-// the untwist of register q, with the inverse's normalisation and Torus
-// scale folded in: 2^23 for N = 1024 Torus32, 2^54 for N = 2048 Torus64;
-// power-of-two scaling commutes with every rounding)
+// e^{i pi n2 / 32} (the compile-time part of the N = 2048 halves' forward
+// twist) and c_utwq[q] = e^{-i pi ((q mod 8) + 16 (q / 8)) / 64} 2^54 (the
+// compile-time part of the untwist of register q, with the normalisation and
+// the Torus64 scale; power-of-two scaling commutes with every rounding)
 static __constant__ double2 c_tw32[16];
 static __constant__ double2 c_utwq[16];
 
-// Where register q of `lane` lands after the lvl1 transforms: frequency bin
+// Where register q of `lane` lands after such a half: frequency bin
 // (forward) or coefficient (inverse) k2 + 16 m + 256 b with k2 = lane & 15,
 // m = (q & 7) + 8 (lane >> 4), b = q >> 3.
 __device__ __forceinline__ int ffnt_pos(int lane, int q)
@@ -234,75 +232,6 @@ __device__ __forceinline__ void radix2_pair(double2 (&v)[16], int h)
         v[j] = cadd(e0, t);
         v[8 + j] = csub(e0, t);
     }
-}
-
-// Forward FFNT of one folded polynomial: in v[n2] = d[n] + i d[n + 512] for
-// n = lane + 32 n2; out v[q] = bin ffnt_pos(lane, q).  (Storing the bins
-// from inside the radix-2 stage keeps fewer registers live but measured
-// slower.)  The twist
-// psi^n = psi^lane psi^{32 n2} is split into a compile-time factor (before
-// the 16-point DFT) and a per-lane factor merged with the w512^{lane k2}
-// twiddle: lane_sign psi^{lane (1 + 4 k2)}, generated by recurrence from two
-// table reads.
-__device__ __forceinline__ void ffnt_forward_warp(double2 (&v)[16], double2* tile,
-                                                  const double2* psi_s, int lane)
-{
-#pragma unroll
-    for (int n2 = 1; n2 < 16; n2++) v[n2] = cmul(v[n2], c_tw32[n2]);
-    dft16<1>(v);
-    const double sg = lane_sign(lane);
-    double2 t = psi_s[psi_pos((uint32_t)lane)];
-    t.x *= sg;
-    t.y *= sg;
-    const double2 st = psi_s[psi_pos(4u * (uint32_t)lane)];
-#pragma unroll
-    for (int k2 = 0; k2 < 16; k2++) {
-        v[k2] = cmul(v[k2], t);
-        if (k2 < 15) t = cmul(t, st);
-    }
-#pragma unroll
-    for (int k2 = 0; k2 < 16; k2++) tile[k2 * 33 + lane] = v[k2];
-    __syncwarp();
-    const int k2 = lane & 15, h = lane >> 4;
-#pragma unroll
-    for (int m = 0; m < 16; m++) v[m] = tile[k2 * 33 + h + 2 * m];
-    __syncwarp();
-    dft16<1>(v);
-    radix2_pair<1>(v, h);
-}
-
-// Inverse FFNT: in v[n2] = Z[lane + 32 n2] (natural bins); out v[q] holds
-// z'[n] conj(psi^n) 2^23 for n = ffnt_pos(lane, q): untwisted and in Torus32
-// units before rounding (2^23 = 2^32 / 512).
-__device__ __forceinline__ void ffnt_inverse_warp(double2 (&v)[16], double2* tile,
-                                                  const double2* psi_s, int lane)
-{
-    dft16<-1>(v);
-    {
-        const double sg = lane_sign(lane);
-        const double2 st = psi_s[psi_pos(4u * (uint32_t)lane)];  // w512^{lane} = psi^{4 lane}
-        double2 t = make_double2(st.x * sg, st.y * sg);
-        v[0].x *= sg;
-        v[0].y *= sg;
-#pragma unroll
-        for (int k2 = 1; k2 < 16; k2++) {
-            v[k2] = cmulc(v[k2], t);
-            if (k2 < 15) t = cmul(t, st);
-        }
-    }
-#pragma unroll
-    for (int k2 = 0; k2 < 16; k2++) tile[k2 * 33 + lane] = v[k2];
-    __syncwarp();
-    const int k2 = lane & 15, h = lane >> 4;
-#pragma unroll
-    for (int m = 0; m < 16; m++) v[m] = tile[k2 * 33 + h + 2 * m];
-    __syncwarp();
-    dft16<-1>(v);
-    radix2_pair<-1>(v, h);
-    // untwist conj(psi^{k2 + 128 h}) conj(psi^{16 (q mod 8) + 256 (q / 8)}) 2^23
-    const double2 u = psi_s[psi_pos((uint32_t)(k2 + 128 * h))];
-#pragma unroll
-    for (int q = 0; q < 16; q++) v[q] = cmul(cmulc(v[q], u), c_utwq[q]);
 }
 
 // ---------------------------------------------------------------------------
