@@ -44,6 +44,8 @@ constexpr uint64_t kDecOffset2 = (512ull << 54) + (512ull << 44) + (512ull << 34
                                  (512ull << 24) + (1ull << 23);
 constexpr size_t kTrgswF2 = 8 * 2 * 1024;  // double2 per Fourier TRGSW<lvl2>
 
+constexpr unsigned kPrefetchCtas2 = 148;  // CTAs that share a step's prefetch
+
 template <int G>
 constexpr size_t br2_smem_bytes()
 {
@@ -109,10 +111,62 @@ __device__ __forceinline__ uint64_t to_torus64(double x)
     return (i >> 63) ? 0ull - v : v;
 }
 
+// Products of one bin: o[j] += sum over the four digit rows of input polynomial
+// c (spectra Z) with the key; bk: the bin's words of the first of these rows,
+// both output polynomials side by side (one 256-bit load).  KeyBundle: FFNT(H)
+// of row (c, d) is 2^{-10 (d + 1)} on polynomial c, then the three keys times
+// their factors X^a - 1.
+template <bool KB>
+__device__ __forceinline__ void products(double2 (&o)[2], const double2 (&Z)[4], const double2 (&fac)[3],
+                                         const double2* bk, int c)
+{
+    if constexpr (KB) {
+        double2 h = c ? o[1] : o[0];
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            const double sc = d == 0 ? 0x1p-10 : d == 1 ? 0x1p-20 : d == 2 ? 0x1p-30 : 0x1p-40;
+            h.x = fma(Z[d].x, sc, h.x);
+            h.y = fma(Z[d].y, sc, h.y);
+        }
+        if (c)
+            o[1] = h;
+        else
+            o[0] = h;
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            double2 s0 = make_double2(0.0, 0.0), s1 = s0;
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                double2 k0, k1;
+                key_pair(k0, k1, bk + e * kTrgswF2 + d * 2048);
+                s0 = cfma(s0, Z[d], k0);
+                s1 = cfma(s1, Z[d], k1);
+            }
+            o[0] = cfma(o[0], fac[e], s0);
+            o[1] = cfma(o[1], fac[e], s1);
+        }
+    } else {
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            double2 k0, k1;
+            key_pair(k0, k1, bk + d * 2048);
+            o[0] = cfma(o[0], Z[d], k0);
+            o[1] = cfma(o[1], Z[d], k1);
+        }
+    }
+}
+
 // One CTA per SM (launch bound 1, and at least 120 KB of shared memory
 // requested): the transforms and the MAC want more than the 128 registers per
 // thread that two CTAs per SM would leave (2048 lanes 70.1 -> 66.2 ms, 148
 // lanes 9.2 -> 4.7 ms against two one-lane CTAs per SM).
+// What bounds it: the step's 786 KB of key rows from L2, about 47 bytes per clock
+// in the MAC, half of the step, and in the rest FP64 instructions with three
+// register operands.  Reading both output polynomials' words in one load and
+// bringing the rows of the step after next into the L2 (the 250 MB key does not
+// stay there): 817 lanes 26.3 -> 24.1 ms, one lane (clusters) 4.1 -> 3.8 ms.
+// Measured and not kept: a quarter of a chunk's words copied into shared memory
+// under the transforms with cp.async (29.6 and 4.7 ms).
 template <bool KB, int G>
 __global__ void __launch_bounds__(G * 256, 1)
     k_br2_fp64(const uint32_t* __restrict__ lane_in, int lanes, uint64_t mu,
@@ -162,6 +216,11 @@ __global__ void __launch_bounds__(G * 256, 1)
         // MAC accumulators: [combo][j][bin half]; combo = (pair index, lane)
         double2 out[2][2][2];
         const double2* bk = bkf + (size_t)p * (KB ? 3 : 1) * kTrgswF2;
+        // the key does not stay in the L2: bring in the step after next
+        if (tid == 0 && p + 2 < nsteps)
+            prefetch_part(bk + 2 * (KB ? 3 : 1) * kTrgswF2, (KB ? 3 : 1) * kTrgswF2 * sizeof(double2),
+                          blockIdx.x % kPrefetchCtas2,
+                          gridDim.x < kPrefetchCtas2 ? gridDim.x : kPrefetchCtas2);
 #pragma unroll 1
         for (int c = 0; c < 2; c++) {
             // ---- F: digits of input polynomial c, row d, parity par
@@ -230,41 +289,12 @@ __global__ void __launch_bounds__(G * 256, 1)
                         const double2 wo = cmul(sl[(2 * d + 1) * kSlotStride + k], w4);
                         Z[d] = h ? csub(E, wo) : cadd(E, wo);
                     }
+                    double2 o[2];
 #pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        double2 o = c ? out[q][j][h] : make_double2(0.0, 0.0);
-                        if (KB) {
-                            double2 s0 = make_double2(0.0, 0.0), s1 = s0, s2 = s0;
-#pragma unroll
-                            for (int d = 0; d < 4; d++) {
-                                const int r = c * 4 + d;
-                                const size_t ki = ((size_t)r * 2 + j) * 1024 + bin;
-                                s0 = cfma(s0, Z[d], __ldg(&bk[0 * kTrgswF2 + ki]));
-                                s1 = cfma(s1, Z[d], __ldg(&bk[1 * kTrgswF2 + ki]));
-                                s2 = cfma(s2, Z[d], __ldg(&bk[2 * kTrgswF2 + ki]));
-                            }
-                            if (j == c) {
-                                // FFNT(H) of row (c, d) = 2^{-10 (d + 1)}
-#pragma unroll
-                                for (int d = 0; d < 4; d++) {
-                                    const double sc = d == 0 ? 0x1p-10 : d == 1 ? 0x1p-20
-                                                    : d == 2 ? 0x1p-30 : 0x1p-40;
-                                    o.x = fma(Z[d].x, sc, o.x);
-                                    o.y = fma(Z[d].y, sc, o.y);
-                                }
-                            }
-                            o = cfma(o, fac[h][0], s0);
-                            o = cfma(o, fac[h][1], s1);
-                            o = cfma(o, fac[h][2], s2);
-                        } else {
-#pragma unroll
-                            for (int d = 0; d < 4; d++) {
-                                const int r = c * 4 + d;
-                                o = cfma(o, Z[d], __ldg(&bk[((size_t)r * 2 + j) * 1024 + bin]));
-                            }
-                        }
-                        out[q][j][h] = o;
-                    }
+                    for (int j = 0; j < 2; j++) o[j] = c ? out[q][j][h] : make_double2(0.0, 0.0);
+                    products<KB>(o, Z, fac[h], &bk[(size_t)(c * 4) * 2048 + 2 * bin], c);
+                    out[q][0][h] = o[0];
+                    out[q][1][h] = o[1];
                 }
                 if (c == 1) {
                     // inverse radix-2 split into slots (j, parity) of this lane;
@@ -353,11 +383,12 @@ __global__ void __launch_bounds__(64) k_bk2_to_fft(const uint64_t* __restrict__ 
 #pragma unroll
     for (int q = 0; q < 16; q++) slots[par][ffnt_pos(lane, q)] = v[q];
     __syncthreads();
-    double2* dst = out + (size_t)poly * 1024;
+    // bins of the two polynomials of a row interleaved
+    double2* dst = out + (size_t)(poly >> 1) * 2048 + (poly & 1);
     for (int k = threadIdx.x; k < 512; k += 64) {
         const double2 wo = cmul(slots[1][k], psi2_at<false>(psi2, 4u * k));
-        dst[k] = cadd(slots[0][k], wo);
-        dst[k + 512] = csub(slots[0][k], wo);
+        dst[2 * k] = cadd(slots[0][k], wo);
+        dst[2 * (k + 512)] = csub(slots[0][k], wo);
     }
 }
 
@@ -440,6 +471,11 @@ __global__ void __launch_bounds__(256, 1)
     for (int p = 0; p < nsteps; p++) {
         double2 out[2][2];  // [j][bin half] of this thread's bin pair
         const double2* bk = bkf + (size_t)p * (KB ? 3 : 1) * kTrgswF2;
+        // the key does not stay in the L2: bring in the step after next
+        if (tid == 0 && p + 2 < nsteps)
+            prefetch_part(bk + 2 * (KB ? 3 : 1) * kTrgswF2, (KB ? 3 : 1) * kTrgswF2 * sizeof(double2),
+                          blockIdx.x % kPrefetchCtas2,
+                          gridDim.x < kPrefetchCtas2 ? gridDim.x : kPrefetchCtas2);
 #pragma unroll 1
         for (int c = 0; c < 2; c++) {
             // ---- F (every rank): digits of input polynomial c, row d, parity par
@@ -504,40 +540,12 @@ __global__ void __launch_bounds__(256, 1)
                         const double2 wo = cmul(spec[(2 * d + 1) * kSlotStride + k], w4);
                         Z[d] = h ? csub(E, wo) : cadd(E, wo);
                     }
+                    double2 o[2];
 #pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        double2 o = c ? out[j][h] : make_double2(0.0, 0.0);
-                        if (KB) {
-                            double2 s0 = make_double2(0.0, 0.0), s1 = s0, s2 = s0;
-#pragma unroll
-                            for (int d = 0; d < 4; d++) {
-                                const int r = c * 4 + d;
-                                const size_t ki = ((size_t)r * 2 + j) * 1024 + bin;
-                                s0 = cfma(s0, Z[d], __ldg(&bk[0 * kTrgswF2 + ki]));
-                                s1 = cfma(s1, Z[d], __ldg(&bk[1 * kTrgswF2 + ki]));
-                                s2 = cfma(s2, Z[d], __ldg(&bk[2 * kTrgswF2 + ki]));
-                            }
-                            if (j == c) {
-#pragma unroll
-                                for (int d = 0; d < 4; d++) {
-                                    const double sc = d == 0 ? 0x1p-10 : d == 1 ? 0x1p-20
-                                                    : d == 2 ? 0x1p-30 : 0x1p-40;
-                                    o.x = fma(Z[d].x, sc, o.x);
-                                    o.y = fma(Z[d].y, sc, o.y);
-                                }
-                            }
-                            o = cfma(o, fac[h][0], s0);
-                            o = cfma(o, fac[h][1], s1);
-                            o = cfma(o, fac[h][2], s2);
-                        } else {
-#pragma unroll
-                            for (int d = 0; d < 4; d++) {
-                                const int r = c * 4 + d;
-                                o = cfma(o, Z[d], __ldg(&bk[((size_t)r * 2 + j) * 1024 + bin]));
-                            }
-                        }
-                        out[j][h] = o;
-                    }
+                    for (int j = 0; j < 2; j++) o[j] = c ? out[j][h] : make_double2(0.0, 0.0);
+                    products<KB>(o, Z, fac[h], &bk[(size_t)(c * 4) * 2048 + 2 * bin], c);
+                    out[0][h] = o[0];
+                    out[1][h] = o[1];
                 }
                 if (c == 1) {
 #pragma unroll

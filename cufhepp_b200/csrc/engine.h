@@ -272,7 +272,8 @@ constexpr int kPsi2Entries = 514;  // 513 used, padded to an even count
 
 // FP64 FFNT blind rotation to lvl2 + SampleExtract of `lanes` lvl0 TLWEs;
 // acc_out: TRLWE<lvl2> [lanes][4096], lane_out: TLWE<lvl2> [lanes][2049]
-// (both optional, uint64 words).  bkf: Fourier BK [step][(e)][8][2][1024].
+// (both optional, uint64 words).  bkf: Fourier BK [step][(e)][8][1024][2], the
+// bins of the two output polynomials side by side.
 // in_count > 0: lane l rotates input l mod in_count with test value
 // mu >> (mu_shift (l div in_count)) (several test polynomials in one launch)
 cudaError_t launch_br2_fp64(bool kb, const uint32_t* lane_in, int lanes, uint64_t mu,
