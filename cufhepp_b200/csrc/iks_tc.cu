@@ -12,11 +12,11 @@
 //   res[o] = x_b[o == n0] + sum_c (A B_c)[o] << 8c   mod 2^32
 // K = 14336, |sum| <= 7168 * 128, so INT32 accumulation is exact.
 //
-// The SIMT kernel in keyswitch.cu spends ~800 K integer instructions per key
-// switch; here one 128-gate x 256-column tile is 448 tcgen05.mma.kind::i8
-// (M = 128, N = 256, K = 32) with both operands streamed from pre-swizzled
-// tiles by cp.async.bulk through a 4-stage shared-memory ring, INT32
-// accumulators in TMEM, and the limb recombination in the epilogue.
+// k_iks_prep combines the inputs and packs each digit into two bits; k_iks_gemm
+// expands them to the one-hot bytes in shared memory itself, so the operand A
+// never exists in memory (it was 14 KB per key switch, written once and read by
+// every column tile), and streams the key tiles once for two unit tiles.
+#include "engine.h"
 #include "engine.h"
 #include "tc_util.cuh"
 
@@ -32,24 +32,19 @@ constexpr int kOutPerTile = kNCols / 4;     // 64
 constexpr int kNTiles = (kTlwe0 + kOutPerTile - 1) / kOutPerTile;  // 10
 constexpr int kATile = kMGates * kChunkK;   // 16 KB
 constexpr int kBTile = kNCols * kChunkK;    // 32 KB
-constexpr int kStageBytes = kATile + kBTile;
-constexpr int kStages = 4;
-constexpr size_t kSmem = 1024 + (size_t)kStages * kStageBytes + 256;
 constexpr uint32_t kIdescIks = idesc_i8(kMGates, kNCols);
 constexpr uint32_t kTmemColsIks = 256;
-// MT unit tiles per CTA share every key chunk (MT accumulators of 256 TMEM
-// columns): a stage holds MT A tiles and one B tile.  MT = 2 halves the key
-// bytes streamed per unit, for keys far larger than L2 (private key
-// switching: 2.5 GB per function).
+// Private key switching: MT unit tiles per CTA share every key chunk (MT
+// accumulators of 256 TMEM columns): a stage holds MT A tiles and one B tile.
+// MT = 2 halves the key bytes streamed per unit (2.5 GB per function).
 template <int MT>
-constexpr int iks_stages() { return MT == 1 ? kStages : 3; }
+constexpr int iks_stages() { return MT == 1 ? 4 : 3; }
 template <int MT>
 constexpr size_t iks_smem() { return 1024 + (size_t)iks_stages<MT>() * (MT * kATile + kBTile) + 256; }
 
 // K = (i, j, e) of an input with NIN mask coefficients: NIN * 7 * 2
 template <int NIN>
 constexpr int iks_chunks() { return NIN * kT * 2 / kChunkK; }  // 112 (lvl1), 224 (lvl2)
-constexpr int kK = kN * kT * 2;             // 14336
 constexpr int kChunks = iks_chunks<kN>();
 
 __host__ __device__ constexpr uint32_t iks_offset_tc()
@@ -94,25 +89,51 @@ __global__ void k_iks_key(const uint32_t* __restrict__ ksk, uint8_t* __restrict_
     reinterpret_cast<uint32_t*>(out)[q] = packed;
 }
 
-// one-hot byte pair of digit code (v = code - 2): v = -1 -> +KSK[.][0],
-// v = +1 -> -KSK[.][0], v = -2 -> +KSK[.][1]
-__device__ __forceinline__ uint32_t onehot_pair(uint32_t code)
+// Digits of a chunk (64 (i, j) pairs) of one unit: two-bit codes (v = code - 2),
+// pair 16 w + 4 s + b at bits 8 b + 2 s of word w.  x(i) returns input word i
+// plus the decomposition offset, whose digit j is at bits kTop - 2 j.
+template <int kTop, typename F>
+__device__ __forceinline__ uint4 digit_codes(int kc, F x)
 {
-    const uint32_t b0 = code == 1 ? 0x01u : (code == 3 ? 0xFFu : 0u);
-    const uint32_t b1 = code == 0 ? 0x01u : 0u;
-    return b0 | (b1 << 8);
+    uint32_t w[4] = {0, 0, 0, 0};
+    int i = 64 * kc / kT, j = 64 * kc % kT;
+    auto t = x(i);
+#pragma unroll
+    for (int e = 0; e < 64; e++) {
+        const uint32_t code = (uint32_t)(t >> (kTop - 2 * j)) & 3u;
+        w[e >> 4] |= code << (8 * (e & 3) + 2 * ((e >> 2) & 3));
+        if (++j == kT) {
+            j = 0;
+            if (e < 63) t = x(++i);
+        }
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// one-hot digit tiles of unit u (a lane in mode 0, a gate in mode 1):
-// atiles[u / 128][kc][16 KB], row u % 128; xb[u] = b part; valid[u]
-__global__ void __launch_bounds__(256) k_iks_prep(int mode, Plan plan, const uint32_t* __restrict__ in0,
+constexpr int kPrepUnits = 8;  // per CTA: eight rows' codes of a chunk are 128 bytes
+
+// Rows of the result before the products: zero, with b in the last word.  Not
+// done when dst may overlap the inputs (k_iks_init does it afterwards).
+__device__ __forceinline__ void init_row(uint32_t* row, uint32_t b, int part, int parts)
+{
+    for (int o = part; o < kTlwe0; o += parts) row[o] = o == kTlwe0 - 1 ? b : 0u;
+}
+
+// digit codes of the units (lanes in mode 0, gates in mode 1):
+// codes[u / 128][kc][u % 128]; xb[u] = b part; valid[u]
+__global__ void __launch_bounds__(256) k_iks_prep(int mode, Plan plan, int units,
+                                                  const uint32_t* __restrict__ in0,
                                                   const uint32_t* __restrict__ in1,
                                                   const uint32_t* __restrict__ in2,
                                                   const uint32_t* __restrict__ lane_out,
-                                                  uint8_t* __restrict__ atiles,
-                                                  uint32_t* __restrict__ xb, int* __restrict__ valid)
+                                                  uint4* __restrict__ codes,
+                                                  uint32_t* __restrict__ xb, int* __restrict__ valid,
+                                                  uint32_t* __restrict__ dst,
+                                                  const int32_t* __restrict__ out_idx)
 {
-    const int u = blockIdx.x;
+    const int u = blockIdx.x * kPrepUnits + threadIdx.x % kPrepUnits;
+    const int part = threadIdx.x / kPrepUnits, parts = blockDim.x / kPrepUnits;
+    if (u >= units) return;
     LanePreadd p = {nullptr, nullptr, 0, 0, 0};
     int ok = 0;
     if (mode == 0) {
@@ -126,97 +147,77 @@ __global__ void __launch_bounds__(256) k_iks_prep(int mode, Plan plan, const uin
             ok = 1;
         }
     }
-    if (threadIdx.x == 0) {
-        uint32_t b = 0;
-        if (ok) {
-            b = (uint32_t)p.ca * p.a[kN] + p.off;
-            if (p.cb) b += (uint32_t)p.cb * p.b[kN];
-        }
+    uint32_t b = 0;
+    if (ok) {
+        b = (uint32_t)p.ca * p.a[kN] + p.off;
+        if (p.cb) b += (uint32_t)p.cb * p.b[kN];
+    }
+    if (part == 0) {
         xb[u] = b;
         valid[u] = ok;
     }
-    const uint32_t row = (uint32_t)(u % kMGates);
-    uint8_t* tb = atiles + (size_t)(u / kMGates) * kChunks * kATile;
-    for (int q = threadIdx.x; q < kK / 16; q += blockDim.x) {
-        // 16 bytes = 8 (i, j) pairs x (e = 0, e = 1)
-        uint32_t wv[4] = {0, 0, 0, 0};
-        int ci = -1;
-        uint32_t t = 0;
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const int pr = 8 * q + e, i = pr / kT, j = pr % kT;
-            if (i != ci) {
-                ci = i;
-                uint32_t x = 0;
-                if (ok) {
-                    x = (uint32_t)p.ca * p.a[i];
-                    if (p.cb) x += (uint32_t)p.cb * p.b[i];
-                }
-                t = x + iks_offset_tc();
-            }
-            const uint32_t code = ok ? (t >> (30 - 2 * j)) & 3u : 2u;  // v = code - 2
-            wv[e >> 1] |= onehot_pair(code) << (16 * (e & 1));
-        }
-        const int k0 = 16 * q;
-        *reinterpret_cast<uint4*>(tb + (size_t)(k0 / kChunkK) * kATile +
-                                  swz_offset(row, (uint32_t)(k0 % kChunkK))) =
-            make_uint4(wv[0], wv[1], wv[2], wv[3]);
-    }
+    if (!ok) return;
+    if (dst) init_row(dst + (out_idx ? (size_t)out_idx[u] : (size_t)u) * kTlwe0, b, part, parts);
+    for (int kc = part; kc < kChunks; kc += parts)
+        codes[((size_t)(u / kMGates) * kChunks + kc) * kMGates + u % kMGates] =
+            digit_codes<30>(kc, [&](int i) {
+                uint32_t x = (uint32_t)p.ca * p.a[i];
+                if (p.cb) x += (uint32_t)p.cb * p.b[i];
+                return x + iks_offset_tc();
+            });
 }
 
-// lvl02 gates: one-hot digit tiles of gate u from its lane outputs at lvl2
+// lvl02 gates: the digit codes of gate u from its lane outputs at lvl2
 // (uint64 TLWE<lvl2>), combined as binary -> lane0, Mux -> lane0 + lane1 +
 // mu2, NMux -> -(lane0 + lane1) - mu2 (src/cufhe_gates_gpu.cu:826-979);
 // xb[u] = the combined b rounded to Torus32 (include/keyswitch_gpu.cuh:33-50).
-__global__ void __launch_bounds__(256) k_iks20_prep(Plan plan, const uint64_t* __restrict__ lane_out,
-                                                    uint8_t* __restrict__ atiles,
-                                                    uint32_t* __restrict__ xb, int* __restrict__ valid)
+__global__ void __launch_bounds__(256) k_iks20_prep(Plan plan, int units,
+                                                    const uint64_t* __restrict__ lane_out,
+                                                    uint4* __restrict__ codes,
+                                                    uint32_t* __restrict__ xb, int* __restrict__ valid,
+                                                    uint32_t* __restrict__ dst)
 {
     constexpr int kCh = iks_chunks<CUFHE_LVL2_N>();
     constexpr int kTl2 = CUFHE_TLWE2_WORDS;
-    const int u = blockIdx.x;
+    const int u = blockIdx.x * kPrepUnits + threadIdx.x % kPrepUnits;
+    const int part = threadIdx.x / kPrepUnits, parts = blockDim.x / kPrepUnits;
+    if (u >= units) return;
     const int l0 = plan_lane0(plan, u);
     const bool ok = l0 >= 0;
     const int op = plan_op(plan, u);
     const uint64_t* A = ok ? lane_out + (size_t)l0 * kTl2 : nullptr;
     const uint64_t* B = (ok && (op == kMux || op == kNMux)) ? A + kTl2 : nullptr;
     const uint64_t neg = op == kNMux ? ~0ull : 0ull;  // x -> -x when set
-    if (threadIdx.x == 0) {
-        uint32_t b = 0;
-        if (ok) {
-            uint64_t x = A[CUFHE_LVL2_N] + (B ? B[CUFHE_LVL2_N] + CUFHE_MU64 : 0ull);
-            x = (x ^ neg) - neg;
-            b = (uint32_t)((x + (1ull << 31)) >> 32);
-        }
+    uint32_t b = 0;
+    if (ok) {
+        uint64_t x = A[CUFHE_LVL2_N] + (B ? B[CUFHE_LVL2_N] + CUFHE_MU64 : 0ull);
+        x = (x ^ neg) - neg;
+        b = (uint32_t)((x + (1ull << 31)) >> 32);
+    }
+    if (part == 0) {
         xb[u] = b;
         valid[u] = ok;
     }
-    const uint32_t row = (uint32_t)(u % kMGates);
-    uint8_t* tb = atiles + (size_t)(u / kMGates) * kCh * kATile;
-    for (int q = threadIdx.x; q < kCh * kChunkK / 16; q += blockDim.x) {
-        uint32_t wv[4] = {0, 0, 0, 0};
-        int ci = -1;
-        uint64_t t = 0;
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const int pr = 8 * q + e, i = pr / kT, j = pr % kT;
-            if (i != ci) {
-                ci = i;
-                uint64_t x = 0;
-                if (ok) {
-                    x = A[i] + (B ? B[i] : 0ull);
-                    x = (x ^ neg) - neg;
-                }
-                t = x + iks20_offset_tc();
-            }
-            const uint32_t code = ok ? (uint32_t)(t >> (62 - 2 * j)) & 3u : 2u;
-            wv[e >> 1] |= onehot_pair(code) << (16 * (e & 1));
-        }
-        const int k0 = 16 * q;
-        *reinterpret_cast<uint4*>(tb + (size_t)(k0 / kChunkK) * kATile +
-                                  swz_offset(row, (uint32_t)(k0 % kChunkK))) =
-            make_uint4(wv[0], wv[1], wv[2], wv[3]);
-    }
+    if (!ok) return;
+    if (dst) init_row(dst + plan_out_row(plan, u) * kTlwe0, b, part, parts);
+    for (int kc = part; kc < kCh; kc += parts)
+        codes[((size_t)(u / kMGates) * kCh + kc) * kMGates + u % kMGates] =
+            digit_codes<62>(kc, [&](int i) {
+                uint64_t x = A[i] + (B ? B[i] : 0ull);
+                x = (x ^ neg) - neg;
+                return x + iks20_offset_tc();
+            });
+}
+
+// init_row of every valid unit, after the inputs have been read
+__global__ void __launch_bounds__(256) k_iks_init(int units, const uint32_t* __restrict__ xb,
+                                                  const int* __restrict__ valid,
+                                                  uint32_t* __restrict__ dst,
+                                                  const int32_t* __restrict__ out_idx)
+{
+    const int u = blockIdx.x;
+    if (u < units && valid[u])
+        init_row(dst + (out_idx ? (size_t)out_idx[u] : (size_t)u) * kTlwe0, xb[u], threadIdx.x, 256);
 }
 
 // ---- private key switching TLWE<lvl2> -> TRLWE<lvl1> as a one-hot GEMM:
@@ -275,7 +276,7 @@ struct OutMap {
 
 // xb (optional) is added to output word OUTW - 1; valid (optional) masks units.
 template <int CH, int NT, int OUTW, int MT = 1>
-__global__ void __launch_bounds__(128, 1) k_iks_gemm(const uint8_t* __restrict__ atiles,
+__global__ void __launch_bounds__(128, 1) k_onehot_gemm(const uint8_t* __restrict__ atiles,
                                                      const uint8_t* __restrict__ btiles,
                                                      const uint32_t* __restrict__ xb,
                                                      const int* __restrict__ valid, int units,
@@ -405,6 +406,211 @@ __global__ void __launch_bounds__(128, 1) k_iks_gemm(const uint8_t* __restrict__
                      "r"(kTmemColsIks * MT));
 }
 
+// ---- the identity key switches' GEMM.  The work is the sequence of chunks of
+// all (pair of unit tiles, column tile) accumulators; CTA c of G takes the c-th
+// G-th of it, so that the last round is as full as the others (4096 units: 160
+// accumulators on 148 SMs) and a single key switch is spread over all SMs (8
+// chunks each instead of 112 in a row).  An accumulator cut between CTAs is
+// summed in dst, mod 2^32 in any order: every CTA adds its part with atomics.
+//   warps 0..7  expand the digit codes of one row per thread into the one-hot
+//               tiles (two tables of four bytes, selected with PRMT), and
+//               afterwards drain the accumulator
+//   warp 8      streams the key tiles (bulk copies) and issues the MMAs
+// What bounds it: the key tiles, 32 KB per chunk from L2 at about 64 B per
+// cycle (512 cycles) against 540 cycles of MMA for two unit tiles.
+// Key switches of 4096 units, prep and GEMM: 264 -> 155 us; of one 76 -> 39 us.
+constexpr int kIksStages = 3;
+constexpr int kIksStageBytes = 2 * kATile + kBTile;
+constexpr int kIksThreads = 288;
+constexpr int kDrainWords = 32 * 33;  // per warp: 32 rows x 32 words, padded
+constexpr size_t kIksSmem = 1024 + (size_t)kIksStages * kIksStageBytes + 8 * kDrainWords * 4 + 128;
+static_assert(kIksSmem <= 232448, "shared memory of the key-switch GEMM");
+
+// 8 one-hot bytes of four digits (set s of a code word): digit v = -1 -> (1, 0),
+// v = +1 -> (-1, 0), v = -2 -> (0, 1), v = 0 -> (0, 0)
+__device__ __forceinline__ uint2 expand4(uint32_t w, int s)
+{
+    const uint32_t sel = ((w >> (2 * s)) & 0x03030303u) * 0x11u + 0x40404040u;
+    return make_uint2(__byte_perm(0xFF000100u, 0x00000001u, sel),
+                      __byte_perm(0xFF000100u, 0x00000001u, sel >> 16));
+}
+
+template <int CH>
+__global__ void __launch_bounds__(kIksThreads, 1)
+    k_iks_gemm(const uint4* __restrict__ codes, const uint8_t* __restrict__ btiles,
+               const int* __restrict__ valid, int units, uint32_t* __restrict__ dst,
+               const int32_t* __restrict__ out_idx, int* __restrict__ err)
+{
+    constexpr int S = kIksStages;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    unsigned char* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
+    uint32_t* drain = reinterpret_cast<uint32_t*>(smem + (size_t)S * kIksStageBytes);
+    uint64_t* full = reinterpret_cast<uint64_t*>(drain + 8 * kDrainWords);
+    uint64_t* empty = full + S;
+    uint64_t* acc_full = empty + S;
+    uint64_t* acc_free = acc_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
+    __shared__ int s_fail;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int gtiles = (units + kMGates - 1) / kMGates, groups = (gtiles + 1) / 2;
+    const long long total = (long long)groups * kNTiles * CH;
+    const int lo = (int)(total * blockIdx.x / gridDim.x);
+    const int hi = (int)(total * (blockIdx.x + 1) / gridDim.x);
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;"
+                     ::"r"(smem_u32(tmem_slot)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        s_fail = 0;
+        for (int s = 0; s < S; s++) {
+            mbar_init(&full[s], 1 + 8);  // the copy's thread and the eight expanding warps
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_free, 8);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 8) {
+        if (lane == 0) {
+            const int n = hi - lo;
+            int filled = 0, committed = 0;  // chunks
+            bool ok = true;
+            auto fill = [&](int it) {
+                const int pos = lo + it, tile = pos / CH, kc = pos % CH;
+                const int s = it % S;
+                mbar_expect_tx(&full[s], (uint32_t)kBTile);
+                bulk_g2s(smem + (size_t)s * kIksStageBytes + 2 * kATile,
+                         btiles + ((size_t)(tile % kNTiles) * CH + kc) * kBTile, kBTile, &full[s]);
+                filled = it + 1;
+            };
+            for (int it = 0; it < S && it < n; it++) fill(it);
+            int seg = 0;
+            for (int it = 0; it < n && ok; it++) {
+                const int pos = lo + it, tile = pos / CH, kc = pos % CH;
+                const int s = it % S;
+                const int mc = gtiles - 2 * (tile / kNTiles) < 2 ? 1 : 2;
+                const bool first = it == 0 || kc == 0;
+                if (first && seg > 0 && !mbar_wait(acc_free, (uint32_t)((seg - 1) & 1))) ok = false;
+                if (ok && !mbar_wait(&full[s], (uint32_t)((it / S) & 1))) ok = false;
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t a0 = smem_u32(smem + (size_t)s * kIksStageBytes);
+                const uint32_t b0 = a0 + 2 * kATile;
+                for (int m = 0; m < mc; m++)
+#pragma unroll
+                    for (int k = 0; k < kChunkK / 32; k++)
+                        tc_mma_i8_ss(tmem + kTmemColsIks * m, desc_kmajor_sw128(a0 + m * kATile + 32 * k),
+                                     desc_kmajor_sw128(b0 + 32 * k), kIdescIks, !first || k != 0);
+                tc_commit(&empty[s]);
+                committed = it + 1;
+                if (kc == CH - 1 || it == n - 1) {
+                    tc_commit(acc_full);
+                    seg++;
+                }
+                // refill the stage of the chunk before once its MMAs are done
+                if (it >= 1 && it + S - 1 < n) {
+                    if (mbar_wait(&empty[(it - 1) % S], (uint32_t)(((it - 1) / S) & 1)))
+                        fill(it + S - 1);
+                    else
+                        ok = false;
+                }
+            }
+            if (!ok) {
+                s_fail = 1;
+                atomicOr(err, 1);
+                // the copies and MMAs in flight end before the memory they use is freed
+                for (int it = committed; it < filled; it++)
+                    mbar_wait(&full[it % S], (uint32_t)((it / S) & 1));
+                if (committed > 0)
+                    mbar_wait(&empty[(committed - 1) % S], (uint32_t)(((committed - 1) / S) & 1));
+            }
+        }
+    } else {
+        const int m = warp >> 2, row = 32 * (warp & 3) + lane;
+        uint32_t* buf = drain + warp * kDrainWords;
+        int seg = 0;
+        bool ok = true;
+        auto load = [&](int it) {
+            const int pos = lo + it, tile = pos / CH, kc = pos % CH, gt = 2 * (tile / kNTiles) + m;
+            return gt < gtiles ? __ldg(&codes[((size_t)gt * CH + kc) * kMGates + row])
+                               : make_uint4(0, 0, 0, 0);
+        };
+        uint4 c = load(0);
+        for (int it = 0; it < hi - lo && ok; it++) {
+            const int pos = lo + it, tile = pos / CH, kc = pos % CH, s = it % S;
+            const int gt = 2 * (tile / kNTiles) + m;
+            const uint4 cur = c;
+            if (it + 1 < hi - lo) c = load(it + 1);
+            if (it >= S && !mbar_wait(&empty[s], (uint32_t)((it / S - 1) & 1))) ok = false;
+            if (gt < gtiles) {
+                unsigned char* a = smem + (size_t)s * kIksStageBytes + m * kATile;
+                const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const uint2 x = expand4(w[q >> 1], 2 * (q & 1)), y = expand4(w[q >> 1], 2 * (q & 1) + 1);
+                    *reinterpret_cast<uint4*>(a + swz_offset((uint32_t)row, 16u * q)) =
+                        make_uint4(x.x, x.y, y.x, y.y);
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read these stores
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+            if (kc == CH - 1 || it == hi - lo - 1) {
+                // ---- drain: recombine the limbs, transpose, add to the rows
+                if (!mbar_wait(acc_full, (uint32_t)(seg & 1))) ok = false;
+                seg++;
+                tc_fence_after();
+                const int u = gt * kMGates + row;
+                const bool live = ok && gt < gtiles && u < units && valid[u];
+                const long long at = live ? (long long)(out_idx ? out_idx[u] : u) * kTlwe0 : -1;
+                const int o0 = (tile % kNTiles) * kOutPerTile;
+                const unsigned any = __ballot_sync(0xffffffffu, live);
+                if (any) {
+#pragma unroll 1
+                    for (int h = 0; h < 2; h++) {
+#pragma unroll
+                        for (int cc = 0; cc < 4; cc++) {
+                            uint32_t v[32];
+                            tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + kTmemColsIks * m +
+                                          128 * h + 32 * cc, v);
+                            tmem_wait_ld();
+#pragma unroll
+                            for (int oo = 0; oo < 8; oo++)
+                                buf[lane * 33 + 8 * cc + oo] = v[4 * oo] + (v[4 * oo + 1] << 8) +
+                                                               (v[4 * oo + 2] << 16) + (v[4 * oo + 3] << 24);
+                        }
+                        __syncwarp();
+                        const int o = o0 + 32 * h + lane;
+#pragma unroll 4
+                        for (int r = 0; r < 32; r++) {
+                            const long long ra = __shfl_sync(0xffffffffu, at, r);
+                            if (ra >= 0 && o < kTlwe0) atomicAdd(dst + ra + o, buf[r * 33 + lane]);
+                        }
+                        __syncwarp();
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_free);
+            }
+        }
+        if (!ok && lane == 0) atomicOr(err, 1);
+    }
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+}
+
 }  // namespace
 
 size_t iks_tc_key_bytes() { return (size_t)kNTiles * kChunks * kBTile; }
@@ -427,16 +633,19 @@ cudaError_t iks20_tc_key_build(const uint32_t* ksk_dev, uint8_t* key_tiles, cuda
     return cudaGetLastError();
 }
 
-static cudaError_t iks_tc_workspace(IksWorkspace& w, int units, int chunks, cudaStream_t st)
+// bytes_per_row: operand bytes of one unit in one chunk (digit codes 16,
+// one-hot tiles of the private key switch 128)
+static cudaError_t iks_tc_workspace(IksWorkspace& w, int units, int chunks, int bytes_per_row,
+                                    cudaStream_t st)
 {
     if ((size_t)units <= w.cap && chunks == w.chunks) return cudaSuccess;
     iks_tc_workspace_free(w);
-    const size_t tiles = (size_t)(units + kMGates - 1) / kMGates;
+    const size_t bytes = (size_t)((units + kMGates - 1) / kMGates) * chunks * kMGates * bytes_per_row;
     cudaError_t e;
-    if ((e = cudaMalloc(&w.atiles, tiles * chunks * kATile)) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&w.atiles, bytes)) != cudaSuccess) return e;
     // zeroed in stream order: the engine's streams are non-blocking, so a
     // memset on the legacy stream could land after the first prep's stores
-    if ((e = cudaMemsetAsync(w.atiles, 0, tiles * chunks * kATile, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(w.atiles, 0, bytes, st)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&w.xb, (size_t)units * 4)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&w.valid, (size_t)units * 4)) != cudaSuccess) return e;
     w.cap = (size_t)units;
@@ -446,7 +655,7 @@ static cudaError_t iks_tc_workspace(IksWorkspace& w, int units, int chunks, cuda
 
 cudaError_t iks_tc_reserve(IksWorkspace& w, int units, bool lvl2, cudaStream_t st)
 {
-    return iks_tc_workspace(w, units, lvl2 ? iks_chunks<CUFHE_LVL2_N>() : kChunks, st);
+    return iks_tc_workspace(w, units, lvl2 ? iks_chunks<CUFHE_LVL2_N>() : kChunks, 16, st);
 }
 
 void iks_tc_workspace_free(IksWorkspace& w)
@@ -462,10 +671,26 @@ static cudaError_t gemm_attr()
 {
     static DeviceAttrFlags attr;
     {
-        const cudaError_t e = set_smem_attr_once(attr, k_iks_gemm<CH, NT, OUTW, MT>, iks_smem<MT>());
+        const cudaError_t e = set_smem_attr_once(attr, k_onehot_gemm<CH, NT, OUTW, MT>, iks_smem<MT>());
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+// the GEMM on as many CTAs as there are SMs, but at least two chunks each
+template <int CH>
+static cudaError_t launch_iks_gemm(const IksWorkspace& w, const uint8_t* key_tiles, int units,
+                                   uint32_t* dst, const int32_t* out_idx, int* err, cudaStream_t st)
+{
+    static DeviceAttrFlags attr;
+    const cudaError_t e = set_smem_attr_once(attr, k_iks_gemm<CH>, kIksSmem);
+    if (e != cudaSuccess) return e;
+    int sms = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    k_iks_gemm<CH><<<sms, kIksThreads, kIksSmem, st>>>(reinterpret_cast<const uint4*>(w.atiles), key_tiles,
+                                                       w.valid, units, dst, out_idx, err);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_iks_tc(int mode, const Plan& plan, const uint32_t* in0, const uint32_t* in1,
@@ -476,16 +701,24 @@ cudaError_t launch_iks_tc(int mode, const Plan& plan, const uint32_t* in0, const
     *launches = 0;
     const int units = mode == 0 ? plan.lanes : plan.count;
     if (units <= 0) return cudaSuccess;
-    cudaError_t e = iks_tc_workspace(w, units, kChunks, st);
-    if (e == cudaSuccess) e = gemm_attr<kChunks, kNTiles, kTlwe0>();
+    cudaError_t e = iks_tc_workspace(w, units, kChunks, 16, st);
     if (e != cudaSuccess) return e;
-    k_iks_prep<<<units, 256, 0, st>>>(mode, plan, in0, in1, in2, lane_out, w.atiles, w.xb, w.valid);
-    const int gtiles = (units + kMGates - 1) / kMGates;
-    const OutMap om = {mode == 1 ? plan.out_idx : nullptr, 0x7fffffff, (size_t)kTlwe0, 0};
-    k_iks_gemm<kChunks, kNTiles, kTlwe0>
-        <<<gtiles * kNTiles, 128, kSmem, st>>>(w.atiles, key_tiles, w.xb, w.valid, units, dst, om, err);
-    *launches = 2;
-    return cudaGetLastError();
+    const int32_t* out_idx = mode == 1 ? plan.out_idx : nullptr;
+    // the rows of dst are cleared before the products are added: with the
+    // digits, unless dst overlaps the inputs (a caller's in-place key switch; the
+    // gates' inputs of mode 0 and dst, the engine's lane buffer, never do)
+    const char* d0 = reinterpret_cast<const char*>(dst);
+    const char* a0 = reinterpret_cast<const char*>(lane_out);
+    const bool inplace = mode == 1 && !out_idx && d0 < a0 + (size_t)plan.lanes * kTlwe1 * 4 &&
+                         a0 < d0 + (size_t)units * kTlwe0 * 4;
+    k_iks_prep<<<(units + kPrepUnits - 1) / kPrepUnits, 256, 0, st>>>(
+        mode, plan, units, in0, in1, in2, lane_out, reinterpret_cast<uint4*>(w.atiles), w.xb, w.valid,
+        inplace ? nullptr : dst, out_idx);
+    if (inplace) k_iks_init<<<units, 256, 0, st>>>(units, w.xb, w.valid, dst, out_idx);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    *launches = inplace ? 3 : 2;
+    return launch_iks_gemm<kChunks>(w, key_tiles, units, dst, out_idx, err, st);
 }
 
 cudaError_t launch_iks20_tc(const Plan& plan, const uint64_t* lane_out, const uint8_t* key_tiles,
@@ -496,16 +729,19 @@ cudaError_t launch_iks20_tc(const Plan& plan, const uint64_t* lane_out, const ui
     *launches = 0;
     const int units = plan.count;
     if (units <= 0) return cudaSuccess;
-    cudaError_t e = iks_tc_workspace(w, units, kCh, st);
-    if (e == cudaSuccess) e = gemm_attr<kCh, kNTiles, kTlwe0>();
+    cudaError_t e = iks_tc_workspace(w, units, kCh, 16, st);
     if (e != cudaSuccess) return e;
-    k_iks20_prep<<<units, 256, 0, st>>>(plan, lane_out, w.atiles, w.xb, w.valid);
-    const int gtiles = (units + kMGates - 1) / kMGates;
-    const OutMap om = {plan.out_idx, 0x7fffffff, (size_t)kTlwe0, 0};
-    k_iks_gemm<kCh, kNTiles, kTlwe0>
-        <<<gtiles * kNTiles, 128, kSmem, st>>>(w.atiles, key_tiles, w.xb, w.valid, units, dst, om, err);
-    *launches = 2;
-    return cudaGetLastError();
+    const char* d0 = reinterpret_cast<const char*>(dst);
+    const char* a0 = reinterpret_cast<const char*>(lane_out);
+    const bool inplace = !plan.out_idx && d0 < a0 + (size_t)plan.lanes * CUFHE_TLWE2_WORDS * 8 &&
+                         a0 < d0 + (size_t)units * kTlwe0 * 4;
+    k_iks20_prep<<<(units + kPrepUnits - 1) / kPrepUnits, 256, 0, st>>>(
+        plan, units, lane_out, reinterpret_cast<uint4*>(w.atiles), w.xb, w.valid, inplace ? nullptr : dst);
+    if (inplace) k_iks_init<<<units, 256, 0, st>>>(units, w.xb, w.valid, dst, nullptr);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    *launches = inplace ? 3 : 2;
+    return launch_iks_gemm<kCh>(w, key_tiles, units, dst, plan.out_idx, err, st);
 }
 
 size_t privks_tc_key_bytes() { return (size_t)kPksNTiles * kPksChunks * kBTile; }
@@ -524,7 +760,7 @@ cudaError_t launch_privks_tc(const uint64_t* tlwe, int units, const uint8_t* key
 {
     *launches = 0;
     if (units <= 0) return cudaSuccess;
-    cudaError_t e = iks_tc_workspace(w, units, kPksChunks, st);
+    cudaError_t e = iks_tc_workspace(w, units, kPksChunks, kChunkK, st);
     constexpr int kMT = 2;  // two unit tiles per CTA share each 2.5 GB key's chunks
     if (e == cudaSuccess) e = gemm_attr<kPksChunks, kPksNTiles, kPksWordsOut, kMT>();
     if (e != cudaSuccess) return e;
@@ -532,7 +768,7 @@ cudaError_t launch_privks_tc(const uint64_t* tlwe, int units, const uint8_t* key
     const int gtiles = (units + kMGates - 1) / kMGates;
     const int ggroups = (gtiles + kMT - 1) / kMT;
     const OutMap om = {nullptr, map.per, map.stride_lo, map.stride_hi};
-    k_iks_gemm<kPksChunks, kPksNTiles, kPksWordsOut, kMT>
+    k_onehot_gemm<kPksChunks, kPksNTiles, kPksWordsOut, kMT>
         <<<ggroups * kPksNTiles, 128, iks_smem<kMT>(), st>>>(w.atiles, key_tiles, nullptr, nullptr,
                                                              units, out, om, err);
     *launches = prep ? 2 : 1;
