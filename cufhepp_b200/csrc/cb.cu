@@ -11,19 +11,19 @@
 
 #include "cufhe_b200.h"
 #include "engine.h"
-#include "fft64.cuh"
+#include "ffnt_tree.cuh"
 
 namespace cufhe {
 
 namespace {
 
 
-// signed digit d (0 = most significant) of an offset Torus32 value, BGBIT bits
+// digit d (0 = most significant) of an offset Torus32 value, BGBIT bits, plus
+// half the base
 template <int L, int BGBIT>
-__device__ __forceinline__ double gadget_digit(uint32_t t, int d)
+__device__ __forceinline__ uint32_t gadget_digit(uint32_t t, int d)
 {
-    return (double)((int32_t)((t >> (32 - (d + 1) * BGBIT)) & ((1u << BGBIT) - 1)) -
-                    (int32_t)(1u << (BGBIT - 1)));
+    return (t >> (32 - (d + 1) * BGBIT)) & ((1u << BGBIT) - 1);
 }
 
 template <int L, int BGBIT>
@@ -34,69 +34,103 @@ constexpr uint32_t gadget_offset()
     return off + (1u << (32 - L * BGBIT - 1));
 }
 
-// One CMUX per CTA, 2L warps: warp r = (input poly j, digit d) transforms its
-// digit row; thread f (bin) multiplies-accumulates with the key; warps 0, 1
-// transform back and add d0.
-template <int L, int BGBIT>
-__global__ void __launch_bounds__(64 * L) k_cmux(CmuxPlan p, const double2* __restrict__ psi,
-                                                 const double2* __restrict__ tw512)
+// G CMUXes per CTA on one key, 2L warps: warp r = (input poly j, digit d)
+// transforms that digit row of each; thread f (bin) multiplies-accumulates with
+// the key, each word read once for all G; the warps share the 2 G inverse
+// transforms and add d0.
+// A row whose digits are all zero is skipped, transform and products: exactly
+// zero is added.  The leaves of a lookup table are constants in eight
+// coefficients of one polynomial and one digit, so at the lowest level, half of
+// a tree's CMUXes, one row of six is left.
+template <int L, int BGBIT, int G>
+__global__ void __launch_bounds__(64 * L, 2) k_cmux(CmuxPlan p, const double2* __restrict__ psi,
+                                                    const double2* __restrict__ tw512)
 {
+    constexpr int W = 2 * L;  // warps, and rows per CMUX
+    constexpr uint32_t kHalf = 1u << (BGBIT - 1);
     extern __shared__ __align__(16) unsigned char cmux_smem[];
-    double2 (*slots)[kSlotStride] = reinterpret_cast<double2 (*)[kSlotStride]>(cmux_smem);
+    double2 (*slots)[kSlotStride] = reinterpret_cast<double2 (*)[kSlotStride]>(cmux_smem);  // [G * 2L]
+    __shared__ int some[G * W];  // the row has a digit that is not zero
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x;
+    const int c = blockIdx.x * G;  // the G CMUXes belong to one group
     const int g = c / p.per, m = c % p.per;
     const size_t node = (size_t)g * p.node_stride_g + (size_t)m * p.node_stride_m;
-    const uint32_t* d0 = p.d0 + node * kTrlwe;
-    const uint32_t* d1 = p.d1 + node * kTrlwe;
     const double2* key = p.trgsw + (size_t)g * p.trgsw_stride;
     uint32_t* out = p.out + ((size_t)g * p.per + m) * kTrlwe;
     constexpr uint32_t kOffG = gadget_offset<L, BGBIT>();
-    {
-        const int j = warp / L, d = warp % L;
+#pragma unroll 1
+    for (int i = 0; i < G; i++) {
+        const int d = warp % L;
+        const size_t at = (node + (size_t)i * p.node_stride_m) * kTrlwe + (warp / L) * kN;
+        const uint32_t *d0 = p.d0 + at, *d1 = p.d1 + at;
         double2 v[16];
+        uint32_t any = 0;
 #pragma unroll
         for (int n2 = 0; n2 < 16; n2++) {
             const int n = lane + 32 * n2;
-            const uint32_t lo = d1[j * kN + n] - d0[j * kN + n];
-            const uint32_t hi = d1[j * kN + n + kHalfN] - d0[j * kN + n + kHalfN];
-            const double2 z = make_double2(gadget_digit<L, BGBIT>(lo + kOffG, d),
-                                           gadget_digit<L, BGBIT>(hi + kOffG, d));
-            v[n2] = cmul(z, __ldg(&psi[n]));
+            const uint32_t lo = gadget_digit<L, BGBIT>(d1[n] - d0[n] + kOffG, d);
+            const uint32_t hi = gadget_digit<L, BGBIT>(d1[n + kHalfN] - d0[n + kHalfN] + kOffG, d);
+            any |= (lo ^ kHalf) | (hi ^ kHalf);
+            v[n2] = make_double2(small_to_double(lo, kHalf), small_to_double(hi, kHalf));
         }
-        fft512_warp<1>(v, slots[warp], tw512, lane);
+        const bool nz = __any_sync(0xffffffffu, any != 0);
+        double2* row = slots[i * W + warp];
+        if (nz) {
 #pragma unroll
-        for (int mm = 0; mm < 16; mm++) slots[warp][(lane & 15) + 16 * mm + 256 * (lane >> 4)] = v[mm];
+            for (int n2 = 0; n2 < 16; n2++) v[n2] = cmul(v[n2], __ldg(&psi[lane + 32 * n2]));
+            fft512_warp<1>(v, row, tw512, lane);
+#pragma unroll
+            for (int mm = 0; mm < 16; mm++) row[(lane & 15) + 16 * mm + 256 * (lane >> 4)] = v[mm];
+        }
+        if (lane == 0) some[i * W + warp] = nz;
     }
     __syncthreads();
-    for (int f = threadIdx.x; f < kHalfN; f += blockDim.x) {
-        double2 o0 = make_double2(0.0, 0.0), o1 = o0;
+    for (int f = threadIdx.x; f < kHalfN; f += 64 * L) {
+        double2 o[G][2];
 #pragma unroll
-        for (int r = 0; r < 2 * L; r++) {
-            const double2 z = slots[r][f];
-            o0 = cfma(o0, z, __ldg(&key[(r * 2 + 0) * kHalfN + f]));
-            o1 = cfma(o1, z, __ldg(&key[(r * 2 + 1) * kHalfN + f]));
+        for (int i = 0; i < G; i++) o[i][0] = o[i][1] = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int r = 0; r < W; r++) {
+            bool use = false;
+#pragma unroll
+            for (int i = 0; i < G; i++) use |= some[i * W + r] != 0;
+            if (!use) continue;
+            const double2 k0 = __ldg(&key[(r * 2 + 0) * kHalfN + f]);
+            const double2 k1 = __ldg(&key[(r * 2 + 1) * kHalfN + f]);
+#pragma unroll
+            for (int i = 0; i < G; i++) {
+                if (some[i * W + r]) {
+                    const double2 z = slots[i * W + r][f];
+                    o[i][0] = cfma(o[i][0], z, k0);
+                    o[i][1] = cfma(o[i][1], z, k1);
+                }
+            }
         }
-        slots[0][f] = o0;  // only this thread reads or writes bin f
-        slots[1][f] = o1;
+        // only this thread reads or writes bin f
+#pragma unroll
+        for (int i = 0; i < G; i++) {
+            slots[i * W + 0][f] = o[i][0];
+            slots[i * W + 1][f] = o[i][1];
+        }
     }
     __syncthreads();
-    if (warp < 2) {
-        const int oj = warp;
+    for (int t = warp; t < 2 * G; t += W) {
+        const int i = t >> 1, oj = t & 1;
+        const uint32_t* d0 = p.d0 + (node + (size_t)i * p.node_stride_m) * kTrlwe + oj * kN;
+        uint32_t* dst = out + (size_t)i * kTrlwe + oj * kN;
+        double2* row = slots[i * W + oj];
         double2 v[16];
 #pragma unroll
-        for (int n2 = 0; n2 < 16; n2++) v[n2] = slots[oj][lane + 32 * n2];
+        for (int n2 = 0; n2 < 16; n2++) v[n2] = row[lane + 32 * n2];
         __syncwarp();
-        fft512_warp<-1>(v, slots[oj], tw512, lane);
+        fft512_warp<-1>(v, row, tw512, lane);
 #pragma unroll
         for (int mm = 0; mm < 16; mm++) {
             const int n = (lane & 15) + 16 * mm + 256 * (lane >> 4);
-            // untwist conj(psi^n), / 512, x 2^32 => x 2^23; llrint as the reference
+            // untwist conj(psi^n), / 512, x 2^32 => x 2^23; rounded as the reference
             const double2 u = cmulc(v[mm], __ldg(&psi[n]));
-            const uint32_t lo = (uint32_t)__double2ll_rn(u.x * 0x1p23);
-            const uint32_t hi = (uint32_t)__double2ll_rn(u.y * 0x1p23);
-            out[oj * kN + n] = d0[oj * kN + n] + lo;
-            out[oj * kN + n + kHalfN] = d0[oj * kN + n + kHalfN] + hi;
+            dst[n] = d0[n] + round_mod32(u.x * 0x1p23);
+            dst[n + kHalfN] = d0[n + kHalfN] + round_mod32(u.y * 0x1p23);
         }
     }
 }
@@ -142,23 +176,31 @@ cudaError_t upload_cb_constants(void)
     return cudaMemcpyToSymbol(c_w32, w, sizeof(w));
 }
 
-template <int L, int BGBIT>
+template <int L, int BGBIT, int G>
 static cudaError_t launch_cmux_t(const CmuxPlan& p, const Fp64Tables& t, cudaStream_t st)
 {
-    constexpr size_t smem = sizeof(double2) * 2 * L * kSlotStride;
+    constexpr size_t smem = sizeof(double2) * G * 2 * L * kSlotStride;
     static DeviceAttrFlags attr;
     {
-        const cudaError_t e = set_smem_attr_once(attr, k_cmux<L, BGBIT>, smem);
+        const cudaError_t e = set_smem_attr_once(attr, k_cmux<L, BGBIT, G>, smem);
         if (e != cudaSuccess) return e;
     }
-    k_cmux<L, BGBIT><<<p.count, 64 * L, smem, st>>>(p, t.psi, t.tw512);
+    k_cmux<L, BGBIT, G><<<p.count / G, 64 * L, smem, st>>>(p, t.psi, t.tw512);
     return cudaGetLastError();
 }
 
 cudaError_t launch_cmux(int gadget, const CmuxPlan& p, const Fp64Tables& t, cudaStream_t st)
 {
     if (p.count <= 0) return cudaSuccess;
-    return gadget == CUFHE_GADGET_CB ? launch_cmux_t<3, 6>(p, t, st) : launch_cmux_t<2, 8>(p, t, st);
+    int sms = 148, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // two CMUXes of a group share the key words once there are enough for two
+    // CTAs of one on every SM; a lone CMUX finishes sooner with the CTA to itself
+    const bool two = p.per % 2 == 0 && p.count % 2 == 0 && p.count > 2 * sms;
+    if (gadget == CUFHE_GADGET_CB)
+        return two ? launch_cmux_t<3, 6, 2>(p, t, st) : launch_cmux_t<3, 6, 1>(p, t, st);
+    return two ? launch_cmux_t<2, 8, 2>(p, t, st) : launch_cmux_t<2, 8, 1>(p, t, st);
 }
 
 cudaError_t launch_lut_leaves(const uint8_t* luts, int q, uint32_t mu, uint32_t* nodes,

@@ -144,3 +144,26 @@ def test_lookup_tables_over_circuit_bootstrapped_bits(cb):
     # output margin: every phase within mu/2 of +-mu
     ph = signed32(client.phase(sk, out.reshape(-1, P.TLWE1_WORDS), 1)).astype(np.float64)
     assert np.abs(np.abs(ph) - P.MU32).max() < P.MU32 / 2
+
+
+@pytest.mark.parametrize("q", [1, 3, 5])
+def test_small_and_repeating_lookup_tables(cb, q):
+    """Few tables (one CMUX per CTA at the upper levels), and entries that repeat
+    or differ in one bit, whose leaf differences have digit rows of zeros."""
+    sk, _ = cb
+    rng = np.random.default_rng(41 + q)
+    luts = rng.integers(0, 256, (q, 256)).astype(np.uint8)
+    luts[0] = 0xA5                      # every difference zero
+    if q > 1:
+        luts[1] = np.arange(256) & 1    # one bit
+    addr = rng.integers(0, 256, q)
+    bits = np.array([(int(addr[t]) >> k) & 1 for t in range(q) for k in range(8)])
+    trgsw = np.stack([client.trgsw_encrypt_g(sk, int(m), seed=43, stream=64 * i, l=3, bgbit=6)
+                      for i, m in enumerate(bits)])
+    d_f = engine.DeviceBuffer(q * 8 * 6 * 2 * 512 * 16)
+    engine.trgsw_to_fft(engine.GADGET_CB, engine.to_device(trgsw), q * 8, d_f)
+    d_o = engine.DeviceBuffer(q * 8 * P.TLWE1_WORDS * 4)
+    engine.lut_eval(luts, d_f, P.MU32, d_o)
+    out = engine.from_device(d_o, (q, 8, P.TLWE1_WORDS))
+    got = client.decrypt_bits(sk, out.reshape(-1, P.TLWE1_WORDS), 1).reshape(q, 8)
+    assert np.array_equal(got, (luts[np.arange(q), addr][:, None] >> np.arange(8)) & 1)
