@@ -63,10 +63,15 @@ __host__ __device__ constexpr uint64_t iks20_offset_tc()
     return off + (1ull << (64 - (1 + CUFHE_LVL20_BASEBIT * CUFHE_LVL20_T)));
 }
 
+// Place of a pair (i, j) in a run of 16: the digit codes of consecutive pairs are
+// consecutive bit pairs of a word, and the expansion takes every fourth.
+__host__ __device__ constexpr int pair_at(int place) { return 4 * (place & 3) + (place >> 2); }
+
 // key tiles [nt][kc][32 KB]: row = o_local * 4 + c, K-major, 128B-swizzled.
 // Key row k (k < KTOT) has OUTW words; rows k >= KTOT and columns o >= OUTW
-// are zero.
-template <int CH, int NT, int OUTW, int KTOT>
+// are zero.  PAIRS: k = (pair, e) with the pairs of each run of 16 in the order
+// of pair_at.
+template <int CH, int NT, int OUTW, int KTOT, bool PAIRS>
 __global__ void k_iks_key(const uint32_t* __restrict__ ksk, uint8_t* __restrict__ out)
 {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -82,35 +87,37 @@ __global__ void k_iks_key(const uint32_t* __restrict__ ksk, uint8_t* __restrict_
     const int c = (int)(row % 4);
     uint32_t packed = 0;
     for (int e = 0; e < 4; e++) {
-        const size_t k = (size_t)kc * kChunkK + kl + e;
+        size_t k = (size_t)kc * kChunkK + kl + e;
+        if (PAIRS) k = (k & ~(size_t)31) + 2 * pair_at((int)(k & 31) >> 1) + (k & 1);
         const int8_t v = (o < OUTW && k < (size_t)KTOT) ? limb(ksk[k * OUTW + o], c) : (int8_t)0;
         packed |= (uint32_t)(uint8_t)v << (8 * e);
     }
     reinterpret_cast<uint32_t*>(out)[q] = packed;
 }
 
-// Digits of a chunk (64 (i, j) pairs) of one unit: two-bit codes (v = code - 2),
-// pair 16 w + 4 s + b at bits 8 b + 2 s of word w.  x(i) returns input word i
-// plus the decomposition offset, whose digit j is at bits kTop - 2 j.
-template <int kTop, typename F>
-__device__ __forceinline__ uint4 digit_codes(int kc, F x)
+// The seven digits of an input word as two-bit codes (v = code - 2), digit j at
+// bits 2 j.  top: the upper 16 bits of the word plus the decomposition offset.
+__device__ __forceinline__ uint32_t digit_field(uint32_t top)
 {
-    uint32_t w[4] = {0, 0, 0, 0};
-    int i = 64 * kc / kT, j = 64 * kc % kT;
-    auto t = x(i);
+    const uint32_t r = __brev(top << 16) & 0x3fffu;  // bit pairs in reverse, each swapped
+    return ((r & 0x1555u) << 1) | ((r >> 1) & 0x1555u);
+}
+
+// The codes of a chunk (64 pairs, 128 bits of the string of fields) of one unit
+__device__ __forceinline__ uint4 chunk_codes(const uint16_t* field, int kc)
+{
+    uint32_t w[4];
 #pragma unroll
-    for (int e = 0; e < 64; e++) {
-        const uint32_t code = (uint32_t)(t >> (kTop - 2 * j)) & 3u;
-        w[e >> 4] |= code << (8 * (e & 3) + 2 * ((e >> 2) & 3));
-        if (++j == kT) {
-            j = 0;
-            if (e < 63) t = x(++i);
-        }
+    for (int q = 0; q < 4; q++) {
+        const int bit = 128 * kc + 32 * q, i = bit / 14;
+        const uint64_t f = (uint64_t)field[i] | (uint64_t)field[i + 1] << 14 |
+                           (uint64_t)field[i + 2] << 28 | (uint64_t)field[i + 3] << 42;
+        w[q] = (uint32_t)(f >> (bit - 14 * i));
     }
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-constexpr int kPrepUnits = 8;  // per CTA: eight rows' codes of a chunk are 128 bytes
+constexpr int kPrepUnits = 8;  // per CTA, one warp each: eight rows' codes of a chunk are 128 bytes
 
 // Rows of the result before the products: zero, with b in the last word.  Not
 // done when dst may overlap the inputs (k_iks_init does it afterwards).
@@ -131,40 +138,48 @@ __global__ void __launch_bounds__(256) k_iks_prep(int mode, Plan plan, int units
                                                   uint32_t* __restrict__ dst,
                                                   const int32_t* __restrict__ out_idx)
 {
-    const int u = blockIdx.x * kPrepUnits + threadIdx.x % kPrepUnits;
-    const int part = threadIdx.x / kPrepUnits, parts = blockDim.x / kPrepUnits;
-    if (u >= units) return;
-    LanePreadd p = {nullptr, nullptr, 0, 0, 0};
-    int ok = 0;
-    if (mode == 0) {
-        p = plan_lane_preadd(plan, u, in0, in1, in2, kTlwe1);
-        ok = 1;
-    } else {
-        const int l0 = plan_lane0(plan, u);
-        if (l0 >= 0) {
-            p = gate_combine(plan_op(plan, u), lane_out + (size_t)l0 * kTlwe1,
-                             lane_out + (size_t)(l0 + 1) * kTlwe1);
+    __shared__ uint16_t field[kPrepUnits][kN + 4];  // four past the end are read, not used
+    // one warp per unit: its digit fields (coalesced)
+    const int here = units - (int)blockIdx.x * kPrepUnits < kPrepUnits
+                         ? units - (int)blockIdx.x * kPrepUnits : kPrepUnits;
+    const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
+    if (wr < here) {
+        const int u = blockIdx.x * kPrepUnits + wr;
+        LanePreadd p = {nullptr, nullptr, 0, 0, 0};
+        int ok = 0;
+        if (mode == 0) {
+            p = plan_lane_preadd(plan, u, in0, in1, in2, kTlwe1);
             ok = 1;
+        } else {
+            const int l0 = plan_lane0(plan, u);
+            if (l0 >= 0) {
+                p = gate_combine(plan_op(plan, u), lane_out + (size_t)l0 * kTlwe1,
+                                 lane_out + (size_t)(l0 + 1) * kTlwe1);
+                ok = 1;
+            }
+        }
+        uint32_t b = 0;
+        if (ok) {
+            const uint32_t* pb = p.cb ? p.b : p.a;  // cb = 0: not used
+#pragma unroll 8
+            for (int i = lane; i < kN; i += 32) {
+                const uint32_t x = (uint32_t)p.ca * p.a[i] + (uint32_t)p.cb * pb[i];
+                field[wr][i] = (uint16_t)digit_field((x + iks_offset_tc()) >> 16);
+            }
+            b = (uint32_t)p.ca * p.a[kN] + (uint32_t)p.cb * pb[kN] + p.off;
+            if (dst) init_row(dst + (out_idx ? (size_t)out_idx[u] : (size_t)u) * kTlwe0, b, lane, 32);
+        }
+        if (lane == 0) {
+            xb[u] = b;
+            valid[u] = ok;
         }
     }
-    uint32_t b = 0;
-    if (ok) {
-        b = (uint32_t)p.ca * p.a[kN] + p.off;
-        if (p.cb) b += (uint32_t)p.cb * p.b[kN];
-    }
-    if (part == 0) {
-        xb[u] = b;
-        valid[u] = ok;
-    }
-    if (!ok) return;
-    if (dst) init_row(dst + (out_idx ? (size_t)out_idx[u] : (size_t)u) * kTlwe0, b, part, parts);
-    for (int kc = part; kc < kChunks; kc += parts)
-        codes[((size_t)(u / kMGates) * kChunks + kc) * kMGates + u % kMGates] =
-            digit_codes<30>(kc, [&](int i) {
-                uint32_t x = (uint32_t)p.ca * p.a[i];
-                if (p.cb) x += (uint32_t)p.cb * p.b[i];
-                return x + iks_offset_tc();
-            });
+    __syncthreads();
+    const int r = threadIdx.x % kPrepUnits, u = blockIdx.x * kPrepUnits + r;
+    if (r < here)
+        for (int kc = threadIdx.x / kPrepUnits; kc < kChunks; kc += 256 / kPrepUnits)
+            codes[((size_t)(u / kMGates) * kChunks + kc) * kMGates + u % kMGates] =
+                chunk_codes(field[r], kc);
 }
 
 // lvl02 gates: the digit codes of gate u from its lane outputs at lvl2
@@ -179,34 +194,42 @@ __global__ void __launch_bounds__(256) k_iks20_prep(Plan plan, int units,
 {
     constexpr int kCh = iks_chunks<CUFHE_LVL2_N>();
     constexpr int kTl2 = CUFHE_TLWE2_WORDS;
-    const int u = blockIdx.x * kPrepUnits + threadIdx.x % kPrepUnits;
-    const int part = threadIdx.x / kPrepUnits, parts = blockDim.x / kPrepUnits;
-    if (u >= units) return;
-    const int l0 = plan_lane0(plan, u);
-    const bool ok = l0 >= 0;
-    const int op = plan_op(plan, u);
-    const uint64_t* A = ok ? lane_out + (size_t)l0 * kTl2 : nullptr;
-    const uint64_t* B = (ok && (op == kMux || op == kNMux)) ? A + kTl2 : nullptr;
-    const uint64_t neg = op == kNMux ? ~0ull : 0ull;  // x -> -x when set
-    uint32_t b = 0;
-    if (ok) {
-        uint64_t x = A[CUFHE_LVL2_N] + (B ? B[CUFHE_LVL2_N] + CUFHE_MU64 : 0ull);
-        x = (x ^ neg) - neg;
-        b = (uint32_t)((x + (1ull << 31)) >> 32);
-    }
-    if (part == 0) {
-        xb[u] = b;
-        valid[u] = ok;
-    }
-    if (!ok) return;
-    if (dst) init_row(dst + plan_out_row(plan, u) * kTlwe0, b, part, parts);
-    for (int kc = part; kc < kCh; kc += parts)
-        codes[((size_t)(u / kMGates) * kCh + kc) * kMGates + u % kMGates] =
-            digit_codes<62>(kc, [&](int i) {
-                uint64_t x = A[i] + (B ? B[i] : 0ull);
+    __shared__ uint16_t field[kPrepUnits][CUFHE_LVL2_N + 4];
+    const int here = units - (int)blockIdx.x * kPrepUnits < kPrepUnits
+                         ? units - (int)blockIdx.x * kPrepUnits : kPrepUnits;
+    const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
+    if (wr < here) {
+        const int u = blockIdx.x * kPrepUnits + wr;
+        const int l0 = plan_lane0(plan, u);
+        uint32_t b = 0;
+        if (l0 >= 0) {
+            const int op = plan_op(plan, u);
+            const uint64_t* A = lane_out + (size_t)l0 * kTl2;
+            const bool two = op == kMux || op == kNMux;
+            const uint64_t* B = two ? A + kTl2 : A;
+            const uint64_t use = two ? 1ull : 0ull;
+            const uint64_t neg = op == kNMux ? ~0ull : 0ull;  // x -> -x when set
+#pragma unroll 8
+            for (int i = lane; i < (int)CUFHE_LVL2_N; i += 32) {
+                uint64_t x = A[i] + use * B[i];
                 x = (x ^ neg) - neg;
-                return x + iks20_offset_tc();
-            });
+                field[wr][i] = (uint16_t)digit_field((uint32_t)((x + iks20_offset_tc()) >> 48));
+            }
+            uint64_t x = A[CUFHE_LVL2_N] + use * (B[CUFHE_LVL2_N] + CUFHE_MU64);
+            x = (x ^ neg) - neg;
+            b = (uint32_t)((x + (1ull << 31)) >> 32);
+            if (dst) init_row(dst + plan_out_row(plan, u) * kTlwe0, b, lane, 32);
+        }
+        if (lane == 0) {
+            xb[u] = b;
+            valid[u] = l0 >= 0;
+        }
+    }
+    __syncthreads();
+    const int r = threadIdx.x % kPrepUnits, u = blockIdx.x * kPrepUnits + r;
+    if (r < here)
+        for (int kc = threadIdx.x / kPrepUnits; kc < kCh; kc += 256 / kPrepUnits)
+            codes[((size_t)(u / kMGates) * kCh + kc) * kMGates + u % kMGates] = chunk_codes(field[r], kc);
 }
 
 // init_row of every valid unit, after the inputs have been read
@@ -416,15 +439,23 @@ __global__ void __launch_bounds__(128, 1) k_onehot_gemm(const uint8_t* __restric
 //               tiles (two tables of four bytes, selected with PRMT), and
 //               afterwards drain the accumulator
 //   warp 8      streams the key tiles (bulk copies) and issues the MMAs
-// What bounds it: the key tiles, 32 KB per chunk from L2 at about 64 B per
-// cycle (512 cycles) against 540 cycles of MMA for two unit tiles.
-// Key switches of 4096 units, prep and GEMM: 264 -> 155 us; of one 76 -> 39 us.
-constexpr int kIksStages = 3;
-constexpr int kIksStageBytes = 2 * kATile + kBTile;
+// A chunk of a pair of tiles takes about 2,100 cycles: 1,024 are MMA (4096 units
+// cannot take less than 63 us of them), and the MMAs' operand reads with the
+// tiles' writes keep shared memory busy for 1,250.  Leaving out the expansion,
+// its stores, the key copies or three quarters of the MMAs in a copy saves 10,
+// 9, 9 and 33 us of 165: no single part is the bound, the hand-over from warp to
+// warp is.
+// Key switches of 4096 units, prep and GEMM: 264 -> 150 us; of one 76 -> 30 us.
+// A 32 KB copy lands about 1.3 us after its issue, hence five key stages; the
+// one-hot tiles are made on the SM and two do (three and four: the same time).
+constexpr int kKeyStages = 5;
+constexpr int kHotStages = 2;
+constexpr int kHotBytes = 2 * kATile;
 constexpr int kIksThreads = 288;
-constexpr int kDrainWords = 32 * 33;  // per warp: 32 rows x 32 words, padded
-constexpr size_t kIksSmem = 1024 + (size_t)kIksStages * kIksStageBytes + 8 * kDrainWords * 4 + 128;
-static_assert(kIksSmem <= 232448, "shared memory of the key-switch GEMM");
+constexpr int kDrainWords = 32 * 33;  // per warp: 32 rows x 32 words, padded; in the one-hot stages
+constexpr size_t kIksSmem = 1024 + (size_t)kHotStages * kHotBytes + (size_t)kKeyStages * kBTile + 256;
+static_assert(kIksSmem <= 232448 && 8 * kDrainWords * 4 <= kHotStages * kHotBytes,
+              "shared memory of the key-switch GEMM");
 
 // 8 one-hot bytes of four digits (set s of a code word): digit v = -1 -> (1, 0),
 // v = +1 -> (-1, 0), v = -2 -> (0, 1), v = 0 -> (0, 0)
@@ -441,14 +472,17 @@ __global__ void __launch_bounds__(kIksThreads, 1)
                const int* __restrict__ valid, int units, uint32_t* __restrict__ dst,
                const int32_t* __restrict__ out_idx, int* __restrict__ err)
 {
-    constexpr int S = kIksStages;
+    constexpr int S = kKeyStages, SA = kHotStages;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
-    unsigned char* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-    uint32_t* drain = reinterpret_cast<uint32_t*>(smem + (size_t)S * kIksStageBytes);
-    uint64_t* full = reinterpret_cast<uint64_t*>(drain + 8 * kDrainWords);
+    unsigned char* hot = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
+    unsigned char* keys = hot + (size_t)SA * kHotBytes;
+    uint32_t* drain = reinterpret_cast<uint32_t*>(hot);
+    uint64_t* full = reinterpret_cast<uint64_t*>(keys + (size_t)S * kBTile);
     uint64_t* empty = full + S;
-    uint64_t* acc_full = empty + S;
+    uint64_t* hot_full = empty + S;
+    uint64_t* hot_empty = hot_full + SA;
+    uint64_t* acc_full = hot_empty + SA;
     uint64_t* acc_free = acc_full + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
     __shared__ int s_fail;
@@ -467,8 +501,12 @@ __global__ void __launch_bounds__(kIksThreads, 1)
     if (tid == 0) {
         s_fail = 0;
         for (int s = 0; s < S; s++) {
-            mbar_init(&full[s], 1 + 8);  // the copy's thread and the eight expanding warps
+            mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < SA; s++) {
+            mbar_init(&hot_full[s], 8);
+            mbar_init(&hot_empty[s], 1);
         }
         mbar_init(acc_full, 1);
         mbar_init(acc_free, 8);
@@ -488,7 +526,7 @@ __global__ void __launch_bounds__(kIksThreads, 1)
                 const int pos = lo + it, tile = pos / CH, kc = pos % CH;
                 const int s = it % S;
                 mbar_expect_tx(&full[s], (uint32_t)kBTile);
-                bulk_g2s(smem + (size_t)s * kIksStageBytes + 2 * kATile,
+                bulk_g2s(keys + (size_t)s * kBTile,
                          btiles + ((size_t)(tile % kNTiles) * CH + kc) * kBTile, kBTile, &full[s]);
                 filled = it + 1;
             };
@@ -501,16 +539,18 @@ __global__ void __launch_bounds__(kIksThreads, 1)
                 const bool first = it == 0 || kc == 0;
                 if (first && seg > 0 && !mbar_wait(acc_free, (uint32_t)((seg - 1) & 1))) ok = false;
                 if (ok && !mbar_wait(&full[s], (uint32_t)((it / S) & 1))) ok = false;
+                if (ok && !mbar_wait(&hot_full[it % SA], (uint32_t)((it / SA) & 1))) ok = false;
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a0 = smem_u32(smem + (size_t)s * kIksStageBytes);
-                const uint32_t b0 = a0 + 2 * kATile;
+                const uint32_t a0 = smem_u32(hot + (size_t)(it % SA) * kHotBytes);
+                const uint32_t b0 = smem_u32(keys + (size_t)s * kBTile);
                 for (int m = 0; m < mc; m++)
 #pragma unroll
                     for (int k = 0; k < kChunkK / 32; k++)
                         tc_mma_i8_ss(tmem + kTmemColsIks * m, desc_kmajor_sw128(a0 + m * kATile + 32 * k),
                                      desc_kmajor_sw128(b0 + 32 * k), kIdescIks, !first || k != 0);
                 tc_commit(&empty[s]);
+                tc_commit(&hot_empty[it % SA]);
                 committed = it + 1;
                 if (kc == CH - 1 || it == n - 1) {
                     tc_commit(acc_full);
@@ -546,13 +586,13 @@ __global__ void __launch_bounds__(kIksThreads, 1)
         };
         uint4 c = load(0);
         for (int it = 0; it < hi - lo && ok; it++) {
-            const int pos = lo + it, tile = pos / CH, kc = pos % CH, s = it % S;
+            const int pos = lo + it, tile = pos / CH, kc = pos % CH, s = it % SA;
             const int gt = 2 * (tile / kNTiles) + m;
             const uint4 cur = c;
             if (it + 1 < hi - lo) c = load(it + 1);
-            if (it >= S && !mbar_wait(&empty[s], (uint32_t)((it / S - 1) & 1))) ok = false;
+            if (it >= SA && !mbar_wait(&hot_empty[s], (uint32_t)((it / SA - 1) & 1))) ok = false;
             if (gt < gtiles) {
-                unsigned char* a = smem + (size_t)s * kIksStageBytes + m * kATile;
+                unsigned char* a = hot + (size_t)s * kHotBytes + m * kATile;
                 const uint32_t w[4] = {cur.x, cur.y, cur.z, cur.w};
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
@@ -563,9 +603,11 @@ __global__ void __launch_bounds__(kIksThreads, 1)
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read these stores
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full[s]);
+            if (lane == 0) mbar_arrive(&hot_full[s]);
             if (kc == CH - 1 || it == hi - lo - 1) {
                 // ---- drain: recombine the limbs, transpose, add to the rows
+                // (through the one-hot stages: every MMA that reads them has ended, and
+                // the next chunk is expanded by warps that have all left the drain)
                 if (!mbar_wait(acc_full, (uint32_t)(seg & 1))) ok = false;
                 seg++;
                 tc_fence_after();
@@ -599,7 +641,7 @@ __global__ void __launch_bounds__(kIksThreads, 1)
                     }
                 }
                 tc_fence_before();
-                __syncwarp();
+                asm volatile("bar.sync 1, 256;" ::: "memory");
                 if (lane == 0) mbar_arrive(acc_free);
             }
         }
@@ -619,7 +661,7 @@ size_t iks20_tc_key_bytes() { return (size_t)kNTiles * iks_chunks<CUFHE_LVL2_N>(
 cudaError_t iks_tc_key_build(const uint32_t* ksk_dev, uint8_t* key_tiles, cudaStream_t st)
 {
     const size_t units = iks_tc_key_bytes() / 4;
-    k_iks_key<kChunks, kNTiles, kTlwe0, kChunks * kChunkK>
+    k_iks_key<kChunks, kNTiles, kTlwe0, kChunks * kChunkK, true>
         <<<(unsigned)((units + 255) / 256), 256, 0, st>>>(ksk_dev, key_tiles);
     return cudaGetLastError();
 }
@@ -628,7 +670,7 @@ cudaError_t iks20_tc_key_build(const uint32_t* ksk_dev, uint8_t* key_tiles, cuda
 {
     const size_t units = iks20_tc_key_bytes() / 4;
     constexpr int kCh2 = iks_chunks<CUFHE_LVL2_N>();
-    k_iks_key<kCh2, kNTiles, kTlwe0, kCh2 * kChunkK>
+    k_iks_key<kCh2, kNTiles, kTlwe0, kCh2 * kChunkK, true>
         <<<(unsigned)((units + 255) / 256), 256, 0, st>>>(ksk_dev, key_tiles);
     return cudaGetLastError();
 }
@@ -749,7 +791,7 @@ size_t privks_tc_key_bytes() { return (size_t)kPksNTiles * kPksChunks * kBTile; 
 cudaError_t privks_tc_key_build(const uint32_t* key_dev, uint8_t* key_tiles, cudaStream_t st)
 {
     const size_t units = privks_tc_key_bytes() / 4;
-    k_iks_key<kPksChunks, kPksNTiles, kPksWordsOut, kPksK>
+    k_iks_key<kPksChunks, kPksNTiles, kPksWordsOut, kPksK, false>
         <<<(unsigned)((units + 255) / 256), 256, 0, st>>>(key_dev, key_tiles);
     return cudaGetLastError();
 }
