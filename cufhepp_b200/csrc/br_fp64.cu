@@ -399,15 +399,6 @@ constexpr size_t one_smem_bytes()
 }
 static_assert(one_smem_bytes<4>() <= kOneSmem && one_smem_bytes<1>() <= 75 * 1024, "CTA layouts");
 
-// the key words of both output polynomials of a row, fetched where the program
-// says so (volatile: not moved down to their use, past the transforms or a
-// barrier)
-__device__ __forceinline__ void key_words(double2 (&k)[2], const double2* p)
-{
-    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-                 : "=d"(k[0].x), "=d"(k[0].y), "=d"(k[1].x), "=d"(k[1].y) : "l"(p));
-}
-
 template <bool KB, int R, int MINB>
 __global__ void __launch_bounds__(256, MINB)
     k_br_fp64_one(const uint32_t* __restrict__ lane_in, int lanes, uint32_t mu,

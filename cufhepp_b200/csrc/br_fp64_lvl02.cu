@@ -111,50 +111,61 @@ __device__ __forceinline__ uint64_t to_torus64(double x)
     return (i >> 63) ? 0ull - v : v;
 }
 
-// Products of one bin: o[j] += sum over the four digit rows of input polynomial
-// c (spectra Z) with the key; bk: the bin's words of the first of these rows,
-// both output polynomials side by side (one 256-bit load).  KeyBundle: FFNT(H)
+// KeyBundle products of one bin: o[j] += sum over the four digit rows of input
+// polynomial c (spectra Z) with the key; bk: the bin's words of the first of
+// these rows, both output polynomials side by side (one 256-bit load).  FFNT(H)
 // of row (c, d) is 2^{-10 (d + 1)} on polynomial c, then the three keys times
 // their factors X^a - 1.
-template <bool KB>
-__device__ __forceinline__ void products(double2 (&o)[2], const double2 (&Z)[4], const double2 (&fac)[3],
-                                         const double2* bk, int c)
+__device__ __forceinline__ void products_kb(double2 (&o)[2], const double2 (&Z)[4], const double2 (&fac)[3],
+                                            const double2* bk, int c)
 {
-    if constexpr (KB) {
-        double2 h = c ? o[1] : o[0];
+    double2 h = c ? o[1] : o[0];
 #pragma unroll
-        for (int d = 0; d < 4; d++) {
-            const double sc = d == 0 ? 0x1p-10 : d == 1 ? 0x1p-20 : d == 2 ? 0x1p-30 : 0x1p-40;
-            h.x = fma(Z[d].x, sc, h.x);
-            h.y = fma(Z[d].y, sc, h.y);
-        }
-        if (c)
-            o[1] = h;
-        else
-            o[0] = h;
+    for (int d = 0; d < 4; d++) {
+        const double sc = d == 0 ? 0x1p-10 : d == 1 ? 0x1p-20 : d == 2 ? 0x1p-30 : 0x1p-40;
+        h.x = fma(Z[d].x, sc, h.x);
+        h.y = fma(Z[d].y, sc, h.y);
+    }
+    if (c)
+        o[1] = h;
+    else
+        o[0] = h;
 #pragma unroll
-        for (int e = 0; e < 3; e++) {
-            double2 s0 = make_double2(0.0, 0.0), s1 = s0;
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                double2 k0, k1;
-                key_pair(k0, k1, bk + e * kTrgswF2 + d * 2048);
-                s0 = cfma(s0, Z[d], k0);
-                s1 = cfma(s1, Z[d], k1);
-            }
-            o[0] = cfma(o[0], fac[e], s0);
-            o[1] = cfma(o[1], fac[e], s1);
-        }
-    } else {
+    for (int e = 0; e < 3; e++) {
+        double2 s0 = make_double2(0.0, 0.0), s1 = s0;
 #pragma unroll
         for (int d = 0; d < 4; d++) {
             double2 k0, k1;
-            key_pair(k0, k1, bk + d * 2048);
-            o[0] = cfma(o[0], Z[d], k0);
-            o[1] = cfma(o[1], Z[d], k1);
+            key_pair(k0, k1, bk + e * kTrgswF2 + d * 2048);
+            s0 = cfma(s0, Z[d], k0);
+            s1 = cfma(s1, Z[d], k1);
         }
+        o[0] = cfma(o[0], fac[e], s0);
+        o[1] = cfma(o[1], fac[e], s1);
     }
 }
+
+// The plain key has 16 words per bin pair and chunk: a thread fetches those of its
+// next pair (both halves, four rows, two outputs) before it needs them, the first
+// ones ahead of the barrier that ends the transforms.
+struct PlainKeys {
+    double2 k[2][4][2];
+    __device__ __forceinline__ void load(const double2* bk)  // the pair's lower bin, first row
+    {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int d = 0; d < 4; d++) key_words(k[h][d], bk + h * 1024 + d * 2048);
+    }
+    __device__ __forceinline__ void products(double2 (&o)[2], const double2 (&Z)[4], int h) const
+    {
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            o[0] = cfma(o[0], Z[d], k[h][d][0]);
+            o[1] = cfma(o[1], Z[d], k[h][d][1]);
+        }
+    }
+};
 
 // One CTA per SM (launch bound 1, and at least 120 KB of shared memory
 // requested): the transforms and the MAC want more than the 128 registers per
@@ -164,7 +175,8 @@ __device__ __forceinline__ void products(double2 (&o)[2], const double2 (&Z)[4],
 // in the MAC, half of the step, and in the rest FP64 instructions with three
 // register operands.  Reading both output polynomials' words in one load and
 // bringing the rows of the step after next into the L2 (the 250 MB key does not
-// stay there): 817 lanes 26.3 -> 24.1 ms, one lane (clusters) 4.1 -> 3.8 ms.
+// stay there): 817 lanes 26.3 -> 24.1 ms, one lane (clusters) 4.1 -> 3.8 ms; plain
+// key, 672 lanes, 32.9 -> 32.5 ms (35.0 with the words loaded where they are used).
 // Measured and not kept: a quarter of a chunk's words copied into shared memory
 // under the transforms with cp.async (29.6 and 4.7 ms).
 template <bool KB, int G>
@@ -253,6 +265,8 @@ __global__ void __launch_bounds__(G * 256, 1)
 #pragma unroll
                 for (int q = 0; q < 16; q++) slot[ffnt_pos(lane, q)] = v[q];
             }
+            PlainKeys pk;
+            if constexpr (!KB) pk.load(&bk[(size_t)(c * 4) * 2048 + 2 * tid]);
             __syncthreads();
 
             // ---- M: radix-2 join + key multiply-accumulate
@@ -292,10 +306,15 @@ __global__ void __launch_bounds__(G * 256, 1)
                     double2 o[2];
 #pragma unroll
                     for (int j = 0; j < 2; j++) o[j] = c ? out[q][j][h] : make_double2(0.0, 0.0);
-                    products<KB>(o, Z, fac[h], &bk[(size_t)(c * 4) * 2048 + 2 * bin], c);
+                    if constexpr (KB)
+                        products_kb(o, Z, fac[h], &bk[(size_t)(c * 4) * 2048 + 2 * bin], c);
+                    else
+                        pk.products(o, Z, h);
                     out[q][0][h] = o[0];
                     out[q][1][h] = o[1];
                 }
+                if constexpr (!KB && G == 1)
+                    if (q == 0) pk.load(&bk[(size_t)(c * 4) * 2048 + 2 * (tid + 256)]);
                 if (c == 1) {
                     // inverse radix-2 split into slots (j, parity) of this lane;
                     // only this thread touches bin k of these slots
@@ -507,6 +526,9 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
                 for (int q = 0; q < 16; q++) slot[ffnt_pos(lane, q)] = v[q];
             }
+            PlainKeys pk;
+            if constexpr (!KB)
+                if (tid < 512 / R) pk.load(&bk[(size_t)(c * 4) * 2048 + 2 * (rank * (512 / R) + tid)]);
             __syncthreads();
 
             // ---- M (rank r): radix-2 join + key MAC of bin pairs [128 r, 128 r + 128)
@@ -543,7 +565,10 @@ __global__ void __launch_bounds__(256, 1)
                     double2 o[2];
 #pragma unroll
                     for (int j = 0; j < 2; j++) o[j] = c ? out[j][h] : make_double2(0.0, 0.0);
-                    products<KB>(o, Z, fac[h], &bk[(size_t)(c * 4) * 2048 + 2 * bin], c);
+                    if constexpr (KB)
+                        products_kb(o, Z, fac[h], &bk[(size_t)(c * 4) * 2048 + 2 * bin], c);
+                    else
+                        pk.products(o, Z, h);
                     out[0][h] = o[0];
                     out[1][h] = o[1];
                 }

@@ -39,6 +39,14 @@ __device__ __forceinline__ void key_pair(double2& k0, double2& k1, const double2
         : "=d"(k0.x), "=d"(k0.y), "=d"(k1.x), "=d"(k1.y) : "l"(p));
 }
 
+// the same, fetched where the program says so (volatile: not moved down to the
+// use, past transforms or a barrier)
+__device__ __forceinline__ void key_words(double2 (&k)[2], const double2* p)
+{
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(k[0].x), "=d"(k[0].y), "=d"(k[1].x), "=d"(k[1].y) : "l"(p));
+}
+
 // Key rows of a later step into L2 (the key shares the L2 with the rest of a
 // gate's data): CTA i of n fetches the i-th part of `bytes`
 __device__ __forceinline__ void prefetch_part(const void* p, uint32_t bytes, uint32_t i, uint32_t n)
