@@ -833,7 +833,7 @@ int autotune_br(int d)
         float best_ms = 1e30f;
         best[i] = 1;
         bound[i] = L;
-        const int cands[] = {1, 2, 4};
+        const int cands[] = {1, 2};
         for (int g : cands) {
             float ms_min = 1e30f;
             for (int rep = 0; rep < 3; rep++) {
