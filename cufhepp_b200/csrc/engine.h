@@ -232,7 +232,7 @@ cudaError_t launch_br_fp64(bool kb, const uint32_t* lane_in, int lanes, uint32_t
 // rotation reads them
 cudaError_t launch_bk_to_fft(const uint32_t* bk, int npolys, const Fp64Tables& t, double2* out,
                              cudaStream_t st, bool pairs);
-// The same rotation with a fixed number of lanes per CTA (1, 2 or 4), for the
+// The same rotation with a fixed number of lanes per CTA (1; else 2), for the
 // autotuner; launch_br_fp64 picks it from the tuned table of the device
 // (br_fp64_set_tuning) or, without one, from the batch size.
 cudaError_t launch_br_fp64_g(int g, bool kb, const uint32_t* lane_in, int lanes, uint32_t mu,
